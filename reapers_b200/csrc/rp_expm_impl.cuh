@@ -254,6 +254,11 @@ constexpr int ACT_KMAX = 40;
 // pieces, go to Pade.
 constexpr double ACT_TERM_US = 0.4, ACT_ROUND_US = 0.35, ACT_ENTRY_US = 0.07, PADE_US = 100.0,
                  PADE_N3_US = 3.7e-3;
+// Largest exponent by which the sum may grow on its way, and the largest of e^(mu/2)
+// (a double ends at e^709): the shifted sum grows like e^(norm of its Hermitian
+// part) although exp(f H) itself may stay below one.  Beyond it: Pade, which
+// scales the matrix as a whole.
+constexpr double ACT_MAX_EXP = 600.0;
 
 // H as its blocks: block b (rows and columns b m ..., the last of order mlast)
 // at blk + b * stride (row-major, leading dimension m), coupling entry sub[b] at
@@ -267,7 +272,8 @@ struct ActionMatrix {
 };
 
 // v, w, y: n entries each in shared memory.  True: y = column 0 of exp(f H);
-// false: too many pieces, the caller takes Pade (blk is left scaled by f).
+// false: too many pieces, or sums beyond a double's range; the caller takes Pade
+// (blk is left scaled by f).
 __device__ inline bool expm_action(const ActionMatrix a, cd f, cd *v, cd *w, cd *y) {
     __shared__ double s_col[32];
     __shared__ cd s_mu;
@@ -292,38 +298,56 @@ __device__ inline bool expm_action(const ActionMatrix a, cd f, cd *v, cd *w, cd 
     }
     __syncthreads();
     const cd mu = s_mu;
-    // 1-norm of A - mu: a warp per column
-    double best = 0.0;
-    for (int j = warp; j < n; j += nw) {
-        const int b = j / m, c = j % m, rows = b == a.nblk - 1 ? a.mlast : m;
-        double s = 0.0;
-        for (int i = lane; i < rows; i += 32) {
-            cd q = a.blk[((size_t)b * m + i) * m + c];
-            if (i == c) q = cd{q.x - mu.x, q.y - mu.y};
-            s += sqrt(q.x * q.x + q.y * q.y);
+    // 1-norm of A - mu (HERM: of its Hermitian part), a warp per column
+    auto norm1 = [&](bool herm) {
+        double best = 0.0;
+        for (int j = warp; j < n; j += nw) {
+            const int b = j / m, c = j % m, rows = b == a.nblk - 1 ? a.mlast : m;
+            const cd *const blk = a.blk + (size_t)b * m * m;
+            double s = 0.0;
+            for (int i = lane; i < rows; i += 32) {
+                cd q = blk[(size_t)i * m + c];
+                if (i == c) q = cd{q.x - mu.x, q.y - mu.y};
+                if (herm) {
+                    cd p = blk[(size_t)c * m + i];
+                    if (i == c) p = cd{p.x - mu.x, p.y - mu.y};
+                    q = cd{0.5 * (q.x + p.x), 0.5 * (q.y - p.y)};
+                }
+                s += sqrt(q.x * q.x + q.y * q.y);
+            }
+            auto coupling = [&](int k) {
+                const cd q = a.sub[k];
+                s += (herm ? 0.5 : 1.0) * sqrt(q.x * q.x + q.y * q.y);
+            };
+            if (lane == 0 && c == m - 1 && b + 1 < a.nblk) coupling(b + 1);
+            if (lane == 0 && herm && c == 0 && b > 0) coupling(b);
+            s = warp_sum(s);
+            // (a NaN stays: fmax would drop it)
+            best = s > best || s != s ? s : best;
         }
-        if (lane == 0 && c == m - 1 && b + 1 < a.nblk) s += sqrt(a.sub[b + 1].x * a.sub[b + 1].x + a.sub[b + 1].y * a.sub[b + 1].y);
-        best = fmax(best, warp_sum(s));
-    }
-    if (lane == 0) s_col[warp] = best;
-    __syncthreads();
-    if (tid == 0) {
+        __syncthreads();
+        if (lane == 0) s_col[warp] = best;
+        __syncthreads();
         double nrm = 0.0;
-        for (int i = 0; i < nw; i++) nrm = fmax(nrm, s_col[i]);
-        s_pieces = 0;
-        if (nrm < 1e6) {                 // (an infinite or NaN norm: Pade)
-            const int pieces = nrm > 2.0 ? (int)ceil(0.5 * nrm) : 1;
-            const double theta = nrm / pieces;
-            int terms = 1;
-            for (double t = theta; t > 2.8e-17 && terms < ACT_KMAX;) t *= theta / ++terms;
-            const int groups = (int)blockDim.x / ACT_T, entries = (m + ACT_T - 1) / ACT_T;
-            const double term = n <= groups && entries <= ACT_Q
-                                    ? ACT_TERM_US
-                                    : (n + groups - 1) / groups * (ACT_ROUND_US + ACT_ENTRY_US * entries);
-            const double n3 = (double)n * n * n;
-            if (term * pieces * terms <= PADE_US + PADE_N3_US * n3) s_pieces = pieces;
-            s_terms = terms;
-        }
+        for (int i = 0; i < nw; i++) nrm = s_col[i] > nrm || s_col[i] != s_col[i] ? s_col[i] : nrm;
+        return nrm;                      // the same in every thread
+    };
+    const double nrm = norm1(false);
+    if (!(nrm < 1e6)) return false;      // (an infinite or NaN norm too)
+    if (nrm > ACT_MAX_EXP && !(norm1(true) <= ACT_MAX_EXP)) return false;
+    if (fabs(mu.x) > 2.0 * ACT_MAX_EXP) return false;
+    if (tid == 0) {
+        const int pieces = nrm > 2.0 ? (int)ceil(0.5 * nrm) : 1;
+        const double theta = nrm / pieces;
+        int terms = 1;
+        for (double t = theta; t > 2.8e-17 && terms < ACT_KMAX;) t *= theta / ++terms;
+        const int groups = (int)blockDim.x / ACT_T, entries = (m + ACT_T - 1) / ACT_T;
+        const double term = n <= groups && entries <= ACT_Q
+                                ? ACT_TERM_US
+                                : (n + groups - 1) / groups * (ACT_ROUND_US + ACT_ENTRY_US * entries);
+        const double n3 = (double)n * n * n;
+        s_pieces = term * pieces * terms <= PADE_US + PADE_N3_US * n3 ? pieces : 0;
+        s_terms = terms;
     }
     __syncthreads();
     const int pieces = s_pieces, terms = s_terms;
@@ -438,10 +462,14 @@ __device__ inline bool expm_action(const ActionMatrix a, cd f, cd *v, cd *w, cd 
             }
         }
     }
-    const double er = exp(mu.x);
+    // e^mu in two halves: y may be as large as e^mu is small
+    const double er = exp(0.5 * mu.x);
     double sn, cs;
     sincos(mu.y, &sn, &cs);
-    for (int i = tid; i < n; i += blockDim.x) y[i] = cmul(cd{er * cs, er * sn}, y[i]);
+    for (int i = tid; i < n; i += blockDim.x) {
+        const cd q = cmul(cd{er * cs, er * sn}, y[i]);
+        y[i] = cd{er * q.x, er * q.y};
+    }
     __syncthreads();
     return true;
 }
