@@ -221,11 +221,9 @@ static void kry_expm_launch(KryWorkspace &ws, int krydim, int cycle, double fr, 
     const size_t pade = (2 * n + 64) * sizeof(double);
     const int action = vecs <= EXPM_SMEM, in_smem = vecs + blocks <= EXPM_SMEM;
     const size_t smem = std::max(pade, in_smem ? vecs + blocks : action ? vecs : 0);
-    static size_t attr = 48 * 1024;
-    if (smem > attr) {
-        RP_CUDA(cudaFuncSetAttribute(k_kry_expm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr = smem;
-    }
+    // always the same value: without it a request just below 48 KB fails too, the
+    // kernel's own static variables counting towards that limit
+    RP_CUDA(cudaFuncSetAttribute(k_kry_expm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EXPM_SMEM));
     k_kry_expm<<<1, 768, smem, st>>>(ws.dev, (cd *)ws.hfull, ws.hcap, (cd *)ws.escratch, krydim, cycle, fr,
                                       fi, in_smem, action, ws.err);
     RP_CUDA(cudaGetLastError());
