@@ -111,6 +111,31 @@ static void row_mark_next(std::vector<RowTerm<float>> &terms, size_t first, size
     }
 }
 
+// CTAs per SM (RPB200_ROW_CTAS, 1 or 2; default 2): the shared memory of an SM
+// (228 KB, 1 KB of it reserved per CTA) is split between them.
+static int row_ctas() {
+    static int ctas = 0;
+    if (!ctas) {
+        const char *e = getenv("RPB200_ROW_CTAS");
+        ctas = (e && atoi(e) == 1) ? 1 : 2;
+    }
+    return ctas;
+}
+
+// Shared memory of a launch beside the ring: the tables, `ndot` projections'
+// sums, and the slack of the swizzle's alignment.
+static size_t row_fixed_bytes(const RowPlan &rp, int ndot) {
+    return rp.terms.size() * sizeof(RowTerm<float>) + rp.groups.size() * sizeof(RowGroup) +
+           (rp.ndiag ? (size_t)rp.ndiag * sizeof(RowDiag) + (size_t)(((1 << rp.logC) + 4) & ~3) * 4 : 0) +
+           (size_t)ROW_NW * ndot * 4 * sizeof(double) + 1024;
+}
+
+// Ring stages that fit beside them, 6 at most; fewer than two do not run.
+static int row_stages(size_t fixed) {
+    const size_t budget = (row_ctas() == 2 ? 113 * 1024 : 227 * 1024) - 64 - 16 * 8;
+    return fixed < budget ? (int)std::min<size_t>(6, (budget - fixed) / (ROW_TILE_BYTES + 16)) : 0;
+}
+
 void rowplan_build(RowPlan &rp, int len, int dtype, const uint64_t *bits, const double *coeff,
                    int64_t nterms, bool any_len, bool fuse_diag, bool merged) {
     rp = RowPlan{};
@@ -119,8 +144,9 @@ void rowplan_build(RowPlan &rp, int len, int dtype, const uint64_t *bits, const 
     const int EPC = 16 / esz;        // elements per 16-byte chunk
     const int logC = log2i(C);
     const int B = logC + 8;
-    // fewer than 128 tiles: the first-generation kernel (unless the caller
-    // only needs the table, as the batched kernel does: one tile suffices)
+    // fewer than 128 tiles: the run or the split row kernel (unless the caller
+    // only needs the table, as the split and the batched kernel do: one tile
+    // suffices)
     if (len < (any_len ? B : B + 7)) return;
     struct T {
         uint32_t x, z;
@@ -193,13 +219,15 @@ void rowplan_build(RowPlan &rp, int len, int dtype, const uint64_t *bits, const 
     // output's own tile (x >> B == 0), with or without terms of its own
     if (rp.ndiag && (rp.groups.empty() || rp.groups[0].xh != 0))
         rp.groups.insert(rp.groups.begin(), RowGroup{0u, 0u, 0u, 0u});
-    if ((int)rp.groups.size() > ROW_MAX_GROUPS) {
+    rp.logC = logC;
+    // (the table alone has the limits above; to run here it also has to leave
+    // room for two stages: about 1400 real strings, or 700 complex ones)
+    if ((int)rp.groups.size() > ROW_MAX_GROUPS || (!any_len && row_stages(row_fixed_bytes(rp, 0)) < 2)) {
         rp = RowPlan{};
         return;
     }
     rp.ok = true;
     rp.B = B;
-    rp.logC = logC;
     rp.ntiles = 1 << (len - B);
     rp.nterms = (int)rp.terms.size();
     // CTAs in flight: two per SM by default (measured fastest on B200:
@@ -562,20 +590,9 @@ template <typename Real>
 static void launch_rows_t(const RowPlan &rp, int len, int dtype, const RowLaunch &l,
                           cudaStream_t st) {
     const bool diag = rp.ndiag > 0;
-    const int C = 128 / (int)sizeof(Cplx<Real>);
-    const size_t fixed = (size_t)rp.nterms * sizeof(RowTerm<float>) +
-                         (size_t)rp.groups.size() * sizeof(RowGroup) +
-                         (diag ? (size_t)rp.ndiag * sizeof(RowDiag) + (size_t)((C + 4) & ~3) * 4 : 0) +
-                         (size_t)ROW_NW * l.ndot * 4 * sizeof(double) + 1024;
-    // CTAs per SM (RPB200_ROW_CTAS, 1 or 2; default 2): the shared memory of
-    // an SM (228 KB, 1 KB of it reserved per CTA) is split between them
-    static int ctas = 0;
-    if (!ctas) {
-        const char *e = getenv("RPB200_ROW_CTAS");
-        ctas = (e && atoi(e) == 1) ? 1 : 2;
-    }
-    const size_t budget = (ctas == 2 ? 113 * 1024 : 227 * 1024) - 64;
-    int S = (int)std::min<size_t>(6, (budget - fixed - 16 * 8) / (ROW_TILE_BYTES + 16));
+    const int ctas = row_ctas();
+    const size_t fixed = row_fixed_bytes(rp, l.ndot);
+    const int S = row_stages(fixed);
     RP_REQUIRE(S >= 2, -2, "Hamiltonian table too large for the row kernel");
     const size_t smem = (size_t)S * ROW_TILE_BYTES + fixed + (size_t)2 * S * sizeof(uint64_t);
     const bool shard = l.shards != nullptr;

@@ -63,8 +63,8 @@ struct RowPlan {
     double alg_bytes_dram = 0;  // (G_w + 1) D s, G_w = distinct x >> (B + log2 window)
 };
 
-// Largest Hamiltonian (terms after splitting, groups) the row kernel stages
-// in shared memory.
+// Largest Hamiltonian (terms after splitting, groups) of a row table; the row
+// kernel takes the tables that leave room for two ring stages (rowplan_build).
 constexpr int ROW_MAX_TERMS = 2048;
 constexpr int ROW_MAX_GROUPS = 1024;
 // Fewest real Z strings worth the fused diagonal (below it they stay terms).

@@ -241,16 +241,31 @@ void splitplan_cut(SplitPlan &p, int parts) {
     }
 }
 
+// Shared memory of a launch beside its stages: a part's tables, the diagonal, and
+// the slack of the swizzle's alignment.
+static size_t split_fixed_bytes(const SplitPlan &p) {
+    return (size_t)p.max_terms * sizeof(RowTerm<float>) + (size_t)p.max_groups * sizeof(RowGroup) +
+           (p.rows.ndiag ? (size_t)p.rows.ndiag * sizeof(RowDiag) + (size_t)(((1 << p.rows.logC) + 4) & ~3) * 4 : 0) +
+           1024;
+}
+
+// Stages that fit beside them with two CTAs per SM, 3 at most; one will do.
+static int split_stages(size_t fixed) {
+    const size_t budget = 113 * 1024 - 64 - 16 * 8;
+    return fixed < budget ? (int)std::min<size_t>(3, (budget - fixed) / (ROW_TILE_BYTES + 16)) : 0;
+}
+
 void splitplan_build(SplitPlan &p, int len, int dtype, const uint64_t *bits, const double *coeff,
                      int64_t nterms) {
     p = SplitPlan{};
     rowplan_build(p.rows, len, dtype, bits, coeff, nterms, true, true);
-    if (!p.rows.ok || p.rows.groups.empty()) return;
+    // (from 128 tiles on a list without a row plan is too long for this kernel too)
+    if (!p.rows.ok || p.rows.groups.empty() || p.rows.ntiles >= 128) return;
     // as many CTAs per tile as fit on the GPU at once, two per SM
     int parts = 1;
     while (parts < 8 && p.rows.ntiles * parts * 2 <= 2 * num_sms()) parts *= 2;
     splitplan_cut(p, parts);
-    p.ok = true;
+    p.ok = split_stages(split_fixed_bytes(p)) >= 1;
 }
 
 void splitplan_upload(SplitPlan &p) {
@@ -272,14 +287,9 @@ void splitplan_free(SplitPlan &p) {
 
 template <typename Real, bool DIAG>
 static void launch_split(const SplitPlan &p, int len, int dtype, const RowLaunch &l, cudaStream_t st) {
-    const int C = 128 / (int)sizeof(Cplx<Real>);
-    const size_t fixed = (size_t)p.max_terms * sizeof(RowTerm<float>) +
-                         (size_t)p.max_groups * sizeof(RowGroup) +
-                         (DIAG ? (size_t)p.rows.ndiag * sizeof(RowDiag) + (size_t)((C + 4) & ~3) * 4 : 0) +
-                         1024;
-    const size_t budget = 113 * 1024 - 64;   // two CTAs per SM
-    const int S = (int)std::min<size_t>(3, (budget - fixed - 16 * 8) / (ROW_TILE_BYTES + 16));
-    RP_REQUIRE(fixed < budget && S >= 1, -2, "Hamiltonian table too large for the split row kernel");
+    const size_t fixed = split_fixed_bytes(p);
+    const int S = split_stages(fixed);
+    RP_REQUIRE(S >= 1, -2, "Hamiltonian table too large for the split row kernel");
     const size_t smem = (size_t)S * ROW_TILE_BYTES + fixed + (size_t)2 * S * sizeof(uint64_t);
     auto kern = k_apply_split<Real, DIAG>;
     static size_t attr_smem = 0;
