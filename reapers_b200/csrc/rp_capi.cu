@@ -101,6 +101,9 @@ static int guarded(F &&f) {
         f();
         return RP_OK;
     } catch (const Error &e) {
+        // (a failed call of the runtime also stays its last error, which the next
+        // launch's check would take for its own)
+        cudaGetLastError();
         set_error(e.code, e.msg);
         return e.code;
     } catch (const std::bad_alloc &) {

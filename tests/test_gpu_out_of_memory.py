@@ -1,0 +1,43 @@
+"""Calls that find no device memory fail alone: the next call runs.  (The sizes
+asked for exceed any GPU's memory, or a filler leaves less than they need.)"""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+import reapers_b200 as rb
+from reapers_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def clean(cuda):
+    _lib.call("rp_workspace_release")
+    torch.cuda.empty_cache()
+    yield
+    _lib.call("rp_workspace_release")
+    torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("entry", ["rp_evolve", "rp_alloc"])
+def test_the_call_after_a_failed_allocation(clean, entry):
+    x = torch.ones(64, dtype=torch.complex128, device="cuda")
+    if entry == "rp_evolve":   # 66 vectors of 64 GB: refused before the state is read
+        ham = rb.Hamiltonian(32, [1], [1.0], "c128")
+        with pytest.raises(rb.RPError) as e:
+            _lib.call("rp_evolve", ham.handle, C.c_void_p(x.data_ptr()), 1.0, 0.0, 64, 1e-12, 0, None)
+        assert e.value.code == -4
+        ham.close()
+    else:
+        p = C.c_void_p()
+        with pytest.raises(rb.RPError):
+            _lib.call("rp_alloc", C.byref(p), 1 << 50)
+    assert rb.norm(x) == 8.0
+    small = rb.Hamiltonian(6, [1], [1.0], "c128")
+    y = torch.empty_like(x)
+    small.apply(y, x)
+    rb.evolve(small, x, 0.5, krydim=4)
+    assert abs(rb.norm(x) - 8.0) < 1e-12 and np.isfinite(rb.norm(y))
+    small.close()
