@@ -83,17 +83,19 @@ void workspace_release(KryWorkspace &ws) {
 void workspace_ensure(KryWorkspace &ws, int len, int dtype, int krydim) {
     if (ws.dev && ws.len == len && ws.dtype == dtype) {
         if (krydim <= ws.krydim) return;
-        // a larger basis for the same state: add vectors, keep the rest
+        // a larger basis for the same state: add vectors, keep the rest (as they
+        // were, when there is no room)
         const size_t vb = ws.D * esize(dtype);
-        while (ws.krydim < krydim) {
-            void *p = nullptr;
-            if (cudaMalloc(&p, vb) != cudaSuccess) {
-                cudaGetLastError();
-                throw Error{-4, "device out of memory for the Krylov workspace"};
-            }
-            ws.u.push_back(p);
-            ws.krydim++;
+        const size_t had = ws.u.size();
+        ws.u.resize((size_t)krydim + 1, nullptr);
+        for (size_t i = had; i < ws.u.size(); i++) {
+            if (cudaMalloc(&ws.u[i], vb) == cudaSuccess) continue;
+            cudaGetLastError();
+            for (size_t k = had; k < i; k++) cudaFree(ws.u[k]);
+            ws.u.resize(had);
+            throw Error{-4, "device out of memory for the Krylov workspace"};
         }
+        ws.krydim = krydim;
         return;
     }
     workspace_release(ws);

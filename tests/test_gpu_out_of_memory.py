@@ -41,3 +41,27 @@ def test_the_call_after_a_failed_allocation(clean, entry):
     rb.evolve(small, x, 0.5, krydim=4)
     assert abs(rb.norm(x) - 8.0) < 1e-12 and np.isfinite(rb.norm(y))
     small.close()
+
+
+def _leave(nbytes):
+    """A tensor that takes all device memory but nbytes."""
+    free = torch.cuda.mem_get_info()[0]
+    return torch.empty(free - nbytes, dtype=torch.uint8, device="cuda")
+
+
+def test_a_basis_that_cannot_grow_gives_back_what_it_took(clean):
+    L, vec = 25, 8 << 25
+    ham = rb.Hamiltonian(L, *rb.syk.xxz_chain(L, 1.0, np.zeros(L)), "c64")
+    x = rb.random_state(L, "c64", seed=1)
+    rb.evolve(ham, x, 0.1, krydim=4, max_iters=1)
+    filler = _leave(int(3.5 * vec))
+    free = torch.cuda.mem_get_info()[0]
+    with pytest.raises(rb.RPError) as e:
+        rb.evolve(ham, x, 0.1, krydim=20, max_iters=1)
+    assert e.value.code == -4
+    assert torch.cuda.mem_get_info()[0] == free
+    before = x.clone()
+    st = rb.evolve(ham, x, 0.1, krydim=5, max_iters=1)   # room for one more
+    assert st["applies"] == 5 and not torch.equal(x, before) and abs(rb.norm(x) - 1.0) < 1e-4
+    del filler
+    ham.close()
