@@ -49,8 +49,14 @@ static void grow_hfull(KryWorkspace &ws, int need, cudaStream_t st) {
     if (need <= ws.hcap) return;
     int cap = std::max(ws.hcap ? ws.hcap : 4 * ws.krydim, 32);
     while (cap < need) cap *= 2;
+    // both before either is replaced: a workspace without room stays as it is
     void *nh = nullptr, *ns = nullptr;
-    RP_CUDA(cudaMalloc(&nh, (size_t)cap * cap * sizeof(cd)));
+    if (cudaMalloc(&nh, (size_t)cap * cap * sizeof(cd)) != cudaSuccess ||
+        cudaMalloc(&ns, ((size_t)2 * cap * cap + expm_scratch_elems(cap)) * sizeof(cd)) != cudaSuccess) {
+        cudaGetLastError();
+        if (nh) cudaFree(nh);
+        throw Error{-4, "device out of memory for the Krylov matrix of " + std::to_string(need) + " rows"};
+    }
     RP_CUDA(cudaMemsetAsync(nh, 0, (size_t)cap * cap * sizeof(cd), st));
     if (ws.hfull) {
         RP_CUDA(cudaMemcpy2DAsync(nh, (size_t)cap * sizeof(cd), ws.hfull,
@@ -59,7 +65,6 @@ static void grow_hfull(KryWorkspace &ws, int need, cudaStream_t st) {
         RP_CUDA(cudaStreamSynchronize(st));
         cudaFree(ws.hfull);
     }
-    RP_CUDA(cudaMalloc(&ns, ((size_t)2 * cap * cap + expm_scratch_elems(cap)) * sizeof(cd)));
     if (ws.escratch) cudaFree(ws.escratch);
     ws.hfull = nh;
     ws.escratch = ns;

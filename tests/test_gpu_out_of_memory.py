@@ -65,3 +65,26 @@ def test_a_basis_that_cannot_grow_gives_back_what_it_took(clean):
     assert st["applies"] == 5 and not torch.equal(x, before) and abs(rb.norm(x) - 1.0) < 1e-4
     del filler
     ham.close()
+
+
+def test_a_krylov_matrix_that_cannot_grow_leaves_the_workspace_whole(clean):
+    """64 vectors: the matrix and its scratch have 256 rows for four cycles (11 MB)
+    and would get 512 (46 MB) in the fifth."""
+    L = 9
+    ham = rb.Hamiltonian(L, *rb.syk.xxz_chain(L, 1.0, np.linspace(-2, 2, L)), "c128")
+    v = rb.random_state(L, "c128", seed=1)
+    first, again, x = v.clone(), v.clone(), v.clone()
+    rb.evolve(ham, first, 30.0, krydim=64, tol=0.0, max_iters=4)
+    filler = _leave(24 << 20)
+    with pytest.raises(rb.RPError) as e:
+        rb.evolve(ham, x, 30.0, krydim=64, tol=0.0, max_iters=5)
+    assert e.value.code == -4
+    rb.evolve(ham, again, 30.0, krydim=64, tol=0.0, max_iters=4)
+    assert torch.equal(again, first)
+    del filler
+    torch.cuda.empty_cache()
+    rb.evolve(ham, x.copy_(v), 30.0, krydim=64, tol=0.0, max_iters=5)
+    _lib.call("rp_workspace_release")
+    rb.evolve(ham, again.copy_(v), 30.0, krydim=64, tol=0.0, max_iters=5)
+    assert torch.equal(again, x)
+    ham.close()
