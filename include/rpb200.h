@@ -260,15 +260,21 @@ typedef struct {
  * the next call.  H receives the m x m Hessenberg matrix, complex interleaved,
  * column-major (2*m*m doubles). */
 int rp_arnoldi(rp_ham_t h, const void *psi, int m, double *H, rp_arnoldi_info_t *info);
-/* m Lanczos steps (2..64) of a Hermitian H from the unit vector psi without
- * reorthogonalisation (the inner loop of Krylov::ground_state,
- * inc/algo.h:180-257): alpha (m doubles), beta (m - 1 doubles); *m_eff < m when
- * beta[*m_eff - 1] is zero (an invariant subspace).  The basis stays on the
- * device for rp_arnoldi_combine. */
-int rp_lanczos(rp_ham_t h, const void *psi, int m, double *alpha, double *beta, int *m_eff);
-/* out = sum_{i < m_eff} coef_i v_i over the last rp_arnoldi or rp_lanczos basis
+/* out = sum_{i < m_eff} coef_i v_i over the last rp_arnoldi basis
  * (coef: 2*m_eff doubles, complex interleaved). */
 int rp_arnoldi_combine(const double *coef, void *out);
+/* m Lanczos steps (2..64) of a Hermitian H from the unit vector vecs[0] without
+ * reorthogonalisation (the inner loop of Krylov::ground_state,
+ * inc/algo.h:180-257): alpha (m doubles), beta (m - 1 doubles); *m_eff < m when
+ * beta[*m_eff - 1] is zero (an invariant subspace).  vecs: m + 1 distinct device
+ * vectors of the caller's, vecs[1..m] overwritten; basis vector j < *m_eff is
+ * vecs[j] / beta[j - 1] (vecs[0] itself for j = 0).  Neither the evolves'
+ * workspace nor the last rp_arnoldi basis is touched. */
+int rp_lanczos(rp_ham_t h, void *const *vecs, int m, double *alpha, double *beta, int *m_eff);
+/* out = sum_{i < nvec} coef_i vecs[i], 1 to 64 vectors, out none of them (coef:
+ * 2*nvec doubles, complex interleaved; summed in FP64, rounded once).  n is even
+ * for complex64. */
+int rp_vec_combine(int dtype, uint64_t n, int nvec, const void *const *vecs, const double *coef, void *out);
 /* For c < ncand: col0[c] = first column of exp((fr[c] + i fi[c]) H), H m x m
  * complex column-major, m <= 1024, ncand <= 64; FP64 Pade-13 on the GPU,
  * one CTA per candidate (col0: 2*m*ncand doubles). */

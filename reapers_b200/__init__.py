@@ -194,40 +194,45 @@ def ground_state(ham, krydim=5, eps=None, maxiter=0, seed=0):
     if eps is None:
         eps = 10 * float(np.finfo(prec).eps)
     v0 = random_state(ham.len, "c64" if ham.dtype == RP_C64 else "c128", seed=seed)
-    cycle = _lanczos if m <= 64 else _lanczos_calls   # rp_lanczos keeps up to 64 vectors
+    vecs = None
     numiter = 0
     while True:
-        try:
-            alpha, beta, ritz = cycle(ham, v0, m)
-        except RPError as e:
-            if e.code != -4 or cycle is _lanczos_calls:
-                raise
-            # no room for the library's m + 2 vectors beside v0
-            cycle = _lanczos_calls
-            continue
+        if m <= 64:   # what rp_lanczos takes
+            if vecs is None:
+                vecs = [torch.empty_like(v0) for _ in range(m)]
+            alpha, beta, ritz = _lanczos(ham, v0, m, vecs)
+        else:
+            alpha, beta, ritz = _lanczos_calls(ham, v0, m)
         evals, evecs = eigh_tridiagonal(np.array(alpha), np.array(beta[:len(alpha) - 1]))
         idx = int(np.argmin(evals))
-        g = ritz(evecs[:, idx], v0)
+        g = ritz(evecs[:, idx])
         scale(g, 1.0 / norm(g))
         numiter += 1
+        if vecs is not None:   # the Ritz vector took the last one's place
+            vecs = [v0] + vecs[:-1]
         v0 = g
         if not (beta and beta[0] > eps and (not maxiter or numiter < maxiter)):
             return float(evals[idx]), g
 
 
-def _lanczos(ham, v0, m):
-    """m Lanczos steps from v0 in one call: (alpha, beta, function giving the
-    basis' combination with real coefficients, which may overwrite `room`)."""
+def _lanczos(ham, v0, m, vecs=None):
+    """m Lanczos steps from v0 in one call, into the m vectors `vecs`: (alpha,
+    beta, function giving the basis' combination with real coefficients, in the
+    last of them)."""
     import torch
+    if vecs is None:
+        vecs = [torch.empty_like(v0) for _ in range(m)]
+    ptrs = (C.c_void_p * (m + 1))(*[_ptr(t).value for t in [v0] + vecs])
     alpha, beta, k = (C.c_double * m)(), (C.c_double * m)(), C.c_int()
-    _lib.call("rp_lanczos", ham.handle, _ptr(v0), m, alpha, beta, C.byref(k))
+    _lib.call("rp_lanczos", ham.handle, ptrs, m, alpha, beta, C.byref(k))
 
-    def ritz(c, room=None):
+    def ritz(c):
         coef = np.zeros(2 * k.value)
         coef[::2] = c
-        g = torch.empty_like(v0) if room is None else room
-        _lib.call("rp_arnoldi_combine", coef.ctypes.data_as(C.POINTER(C.c_double)), _ptr(g))
-        return g
+        coef[2::2] *= 1.0 / np.array(beta[:k.value - 1])   # the vectors are kept unnormalised
+        _lib.call("rp_vec_combine", ham.dtype, v0.numel(), k.value, ptrs,
+                  coef.ctypes.data_as(C.POINTER(C.c_double)), _ptr(vecs[-1]))
+        return vecs[-1]
 
     return alpha[:k.value], beta[:k.value - 1], ritz
 
@@ -253,7 +258,7 @@ def _lanczos_calls(ham, v0, m):
         scale(w, 1.0 / b)
         V.append(w)
 
-    def ritz(c, room=None):
+    def ritz(c):
         g = torch.zeros_like(v0)
         for i, v in enumerate(V):
             axpy(g, float(c[i]), v)

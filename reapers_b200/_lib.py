@@ -87,8 +87,9 @@ _SIGS = {
                             C.POINTER(EvolveStats)]),
     "rp_workspace_release": (C.c_int, []),
     "rp_arnoldi": (C.c_int, [_VP, _VP, C.c_int, C.POINTER(C.c_double), C.POINTER(ArnoldiInfo)]),
-    "rp_lanczos": (C.c_int, [_VP, _VP, C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double),
+    "rp_lanczos": (C.c_int, [_VP, C.POINTER(_VP), C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double),
                              C.POINTER(C.c_int)]),
+    "rp_vec_combine": (C.c_int, [C.c_int, C.c_uint64, C.c_int, C.POINTER(_VP), C.POINTER(C.c_double), _VP]),
     "rp_arnoldi_combine": (C.c_int, [C.POINTER(C.c_double), _VP]),
     "rp_expm_first_column": (C.c_int, [C.c_int, C.POINTER(C.c_double), C.c_int,
                                        C.POINTER(C.c_double), C.POINTER(C.c_double),

@@ -148,7 +148,7 @@ int rp_shutdown(void) {
         std::lock_guard<std::mutex> lk(g_mu);
         if (g_stream) cudaStreamSynchronize(g_stream);
         workspace_release(g_ws);
-        krylov_host_release();
+        krylov_scratch_release();
         pipe_release();
         scratch_release_all();
         dense_handles_release();
@@ -632,12 +632,24 @@ int rp_arnoldi(rp_ham_t h, const void *psi, int m, double *H, rp_arnoldi_info_t 
     });
 }
 
-int rp_lanczos(rp_ham_t h, const void *psi, int m, double *alpha, double *beta, int *m_eff) {
+int rp_lanczos(rp_ham_t h, void *const *vecs, int m, double *alpha, double *beta, int *m_eff) {
     return guarded([&] {
-        RP_REQUIRE(h && alpha && beta && m_eff, RP_E_INVALID, "null argument");
-        check_vec(psi);
-        krylov_lanczos(h->plan, g_ws, psi, m, alpha, beta, g_arn, g_stream);
-        *m_eff = g_arn.m_eff;
+        RP_REQUIRE(h && vecs && alpha && beta && m_eff, RP_E_INVALID, "null argument");
+        for (int i = 0; i <= m && i <= MAX_KRYLOV; i++) check_vec(vecs[i]);
+        *m_eff = krylov_lanczos(h->plan, vecs, m, alpha, beta, g_stream);
+    });
+}
+
+int rp_vec_combine(int dtype, uint64_t n, int nvec, const void *const *vecs, const double *coef, void *out) {
+    return guarded([&] {
+        check_dtype(dtype);
+        RP_REQUIRE(vecs && coef, RP_E_INVALID, "null argument");
+        check_vec(out);
+        for (int i = 0; i < nvec && i < MAX_KRYLOV; i++) {
+            check_vec(vecs[i]);
+            RP_REQUIRE(vecs[i] != out, RP_E_INVALID, "the result may not be one of the vectors");
+        }
+        vec_combine(dtype, n, nvec, vecs, coef, out, g_stream);
     });
 }
 

@@ -248,9 +248,34 @@ static const KryDev &read_back(const KryDev *dev, size_t bytes, cudaStream_t st)
     return *g_host;
 }
 
-void krylov_host_release() {
+// Device state of the Lanczos steps and combinations over the caller's vectors:
+// fixed, and apart from the workspace, whose basis they leave alone.
+struct LanczosScratch {
+    KryDev *dev = nullptr;
+    double *partials = nullptr;          // two sums per CTA
+    unsigned *err = nullptr;
+};
+static LanczosScratch g_lan;
+
+static const LanczosScratch &lanczos_scratch() {
+    if (g_lan.dev) return g_lan;
+    const size_t at = (sizeof(KryDev) + 15) & ~(size_t)15, pb = (size_t)reduce_grid() * 2 * sizeof(double);
+    char *p = nullptr;
+    if (cudaMalloc((void **)&p, at + pb + sizeof(unsigned)) != cudaSuccess) {
+        cudaGetLastError();
+        throw Error{-4, "device out of memory for the Lanczos scratch"};
+    }
+    g_lan.dev = reinterpret_cast<KryDev *>(p);
+    g_lan.partials = reinterpret_cast<double *>(p + at);
+    g_lan.err = reinterpret_cast<unsigned *>(p + at + pb);
+    return g_lan;
+}
+
+void krylov_scratch_release() {
     if (g_host) cudaFreeHost(g_host);
     g_host = nullptr;
+    if (g_lan.dev) cudaFree(g_lan.dev);
+    g_lan = LanczosScratch{};
 }
 
 __global__ void k_kry_err(KryDev *s, const unsigned *err) { s->err = *err; }
@@ -364,40 +389,45 @@ void krylov_arnoldi(const ApplyPlan &plan, KryWorkspace &ws, const void *psi, in
     R.beta = h.beta;
 }
 
-void krylov_lanczos(const ApplyPlan &plan, KryWorkspace &ws, const void *psi, int m, double *alpha,
-                    double *beta, ArnoldiResult &R, cudaStream_t st) {
+int krylov_lanczos(const ApplyPlan &plan, void *const *u, int m, double *alpha, double *beta, cudaStream_t st) {
     RP_REQUIRE(m >= 2 && m <= MAX_KRYLOV, -2, "m must be in [2, 64]");
-    workspace_ensure(ws, plan.len, plan.dtype, m);
-    const uint64_t D = ws.D;
-    KryDev *s = ws.dev;
-    R = ArnoldiResult{};
-    R.m = m;
-    R.beta0 = 1.0;
-    RP_CUDA(cudaMemcpyAsync(ws.u[0], psi, D * esize(plan.dtype), cudaMemcpyDeviceToDevice, st));
-    RP_CUDA(cudaMemsetAsync(ws.err, 0, sizeof(unsigned), st));
+    const LanczosScratch &z = lanczos_scratch();
+    KryDev *s = z.dev;
+    RP_CUDA(cudaMemsetAsync(z.err, 0, sizeof(unsigned), st));
     k_kry_init<<<1, 32, 0, st>>>(s, 1.0);
     k_kry_begin<<<1, 256, 0, st>>>(s, m, 0);
     RP_CUDA(cudaGetLastError());
     for (int j = 0; j < m; j++) {
         ApplyLaunch L;
-        L.in = ws.u[j];
-        L.out = ws.u[j + 1];
+        L.in = u[j];
+        L.out = u[j + 1];
         L.alpha_dev = &s->sigma[j];
         L.active = &s->active;
-        L.err = ws.err;
+        L.err = z.err;
         apply_launch(plan, L, st);
-        lanczos_launch(plan.dtype, D, j ? ws.u[j - 1] : nullptr, ws.u[j], ws.u[j + 1], s, ws.partials, ws.err, j,
-                       j == m - 1, st);
+        lanczos_launch(plan.dtype, 1ull << plan.len, j ? u[j - 1] : nullptr, u[j], u[j + 1], s, z.partials, z.err,
+                       j, j == m - 1, st);
     }
-    k_kry_err<<<1, 1, 0, st>>>(s, ws.err);
+    k_kry_err<<<1, 1, 0, st>>>(s, z.err);
     RP_CUDA(cudaGetLastError());
     const KryDev &h = read_back(s, offsetof(KryDev, coef), st);
-    R.m_eff = h.m_eff;
-    R.sigma.assign(h.sigma, h.sigma + m + 1);
-    for (int j = 0; j < R.m_eff; j++) {
+    for (int j = 0; j < h.m_eff; j++) {
         alpha[j] = h.hacc[2 * j];
         if (j < m - 1) beta[j] = h.hacc[2 * j + 1];
     }
+    return h.m_eff;
+}
+
+void vec_combine(int dtype, uint64_t n, int nvec, const void *const *u, const double *coef, void *out,
+                 cudaStream_t st) {
+    RP_REQUIRE(nvec >= 1 && nvec <= MAX_KRYLOV, -2, "a combination takes 1 to 64 vectors");
+    RP_REQUIRE(dtype == 2 || n % 2 == 0, -2, "a combination of complex64 vectors needs an even length");
+    VecTable tab{};
+    for (int i = 0; i < nvec; i++) tab.p[i] = u[i];
+    double *c = lanczos_scratch().dev->ycoef;
+    RP_CUDA(cudaMemcpyAsync(c, coef, (size_t)nvec * 2 * sizeof(double), cudaMemcpyHostToDevice, st));
+    RP_CUDA(cudaMemsetAsync(out, 0, n * esize(dtype), st));
+    multi_axpy(dtype, n, tab, nvec, nullptr, c, out, st);
 }
 
 void krylov_combine(KryWorkspace &ws, const ArnoldiResult &R, const double *coef, void *out,

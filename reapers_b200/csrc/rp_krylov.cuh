@@ -59,8 +59,9 @@ struct KryWorkspace {
 // (rp_workspace_release frees it).
 void workspace_ensure(KryWorkspace &ws, int len, int dtype, int krydim);
 void workspace_release(KryWorkspace &ws);
-// The pinned host copy of a KryDev that the calls read their results through.
-void krylov_host_release();
+// The pinned host copy of a KryDev that the calls read their results through, and
+// the Lanczos steps' device state.
+void krylov_scratch_release();
 
 // psi <- exp(-(t_imag + i t_real) H) psi, restarted Arnoldi with the
 // Eiermann-Ernst update (inc/algo.h:267-365).  psi is a device vector of the
@@ -94,11 +95,13 @@ struct ArnoldiResult {
 };
 void krylov_arnoldi(const ApplyPlan &plan, KryWorkspace &ws, const void *psi, int m,
                     ArnoldiResult &R, cudaStream_t st);
-// m Lanczos steps from the unit vector psi without reorthogonalisation: alpha
-// (m_eff entries) and beta (m_eff - 1, and a zero after an invariant subspace);
-// the basis stays in the workspace, its scales in R.
-void krylov_lanczos(const ApplyPlan &plan, KryWorkspace &ws, const void *psi, int m, double *alpha,
-                    double *beta, ArnoldiResult &R, cudaStream_t st);
+// m Lanczos steps from the unit vector u[0] without reorthogonalisation, w_{j+1}
+// in u[j + 1]: alpha (returned number of entries) and beta (one less, and a zero
+// after an invariant subspace); v_j = u[j] / beta[j - 1].
+int krylov_lanczos(const ApplyPlan &plan, void *const *u, int m, double *alpha, double *beta, cudaStream_t st);
+// out = sum_i coef_i u[i] (coef complex, host).
+void vec_combine(int dtype, uint64_t n, int nvec, const void *const *u, const double *coef, void *out,
+                 cudaStream_t st);
 // out = sum_{i < m_eff} coef_i v_i over the last basis (coef complex, host).
 void krylov_combine(KryWorkspace &ws, const ArnoldiResult &R, const double *coef, void *out,
                     cudaStream_t st);
