@@ -6,17 +6,19 @@
 // An epoch of training is one cooperative launch.  Per mini-batch every CTA
 // takes the parameters into shared memory, runs its samples forward and
 // backward four at a time (thread = hidden unit x sample) and writes its
-// gradient partial; after a grid barrier the CTAs share the parameters out,
-// sum the partials in a fixed order in FP64 and apply Adam (reproducible);
-// after another the next batch starts.  Loss: mean squared error / 2.
+// gradient partial, products and sums over samples in FP64; after a grid barrier
+// the CTAs share the parameters out, sum the partials in a fixed order and apply
+// Adam (reproducible); after another the next batch starts.  Loss: mean squared
+// error / 2.
 //
 // A batch of 512 is 17 MFLOP: bound by latency (two barriers, the dependent
 // layers), so the design counts launches, host round trips and bank conflicts:
 // weight rows are padded to an odd length in shared memory, the samples stay on
-// the device and an epoch uploads its order alone.  Measured, 9000 samples,
-// batch 512, per epoch: three kernels and a host sync per batch, unpadded rows
-// 2.64 to 4.0 ms (allocations on every call among it) -> 0.46 ms, 0.31 of it the
-// kernel (16 us per batch).
+// the device, an epoch uploads its order alone, and what the FP64 gradient
+// multiplies is converted once per sweep.  Measured, 21 inputs, us per batch of
+// 64 / 512 / 2048 / 8192, three kernels and a host sync per batch -> this: 47.7 /
+// 86.3 / 199 / 458 -> 13.7 / 16.7 / 37.9 / 71.2 (with FP32 sums over a CTA's samples
+// 13.2 / 17.3 / 34.8 / 64.9, and a gradient further from 64 bits than the former).
 #include <cmath>
 #include <vector>
 
@@ -81,6 +83,33 @@ __device__ __forceinline__ MlpShared mlp_carve(const MlpDims &d, float *p) {
     s.dh1 = p, p += MS * HID;
     s.y = p, p += MS * 8;
     s.dy = p;
+    return s;
+}
+
+// The training kernel's FP64 copies of what the gradient multiplies (a value is
+// converted once per sweep, not once per product), and, when it fits, the
+// gradient itself.
+struct MlpShared64 {
+    double *x, *h1, *h2, *dy, *dh2, *dh1, *g;
+};
+
+__host__ __device__ inline size_t mlp_shared_at64(const MlpDims &d) {
+    return (mlp_shared_floats(d) * sizeof(float) + 7) & ~(size_t)7;
+}
+__host__ __device__ inline size_t mlp_shared_doubles(const MlpDims &d) {
+    return (size_t)MS * ((d.in + 3) & ~3) + 4 * MS * HID + MS * 8;
+}
+
+__device__ __forceinline__ MlpShared64 mlp_carve64(const MlpDims &d, void *sm) {
+    double *p = reinterpret_cast<double *>(static_cast<char *>(sm) + mlp_shared_at64(d));
+    MlpShared64 s;
+    s.x = p, p += MS * ((d.in + 3) & ~3);
+    s.h1 = p, p += MS * HID;
+    s.h2 = p, p += MS * HID;
+    s.dh2 = p, p += MS * HID;
+    s.dh1 = p, p += MS * HID;
+    s.dy = p, p += MS * 8;
+    s.g = p;
     return s;
 }
 
@@ -155,15 +184,16 @@ struct MlpSteps {
     int update;                          // 0: the gradient alone, into g
     float lr;
     int step0;                           // Adam steps taken before
-    float *gpart, *loss;                 // [cta][np], [batch]
-    double *lpart;                       // [cta]
+    double *gpart, *lpart;               // [cta][np], [cta]
+    float *loss;                         // [batch]
+    int g_shared;                        // the gradient of several sweeps fits in shared memory
     unsigned *barrier, *err;
 };
 
 __global__ void __launch_bounds__(MT) k_mlp_steps(MlpDims d, const MlpSteps a) {
     extern __shared__ float sm[];
     const MlpShared s = mlp_carve(d, sm);
-    float *G = sm + mlp_shared_floats(d);
+    const MlpShared64 v = mlp_carve64(d, sm);
     __shared__ double red[MS][HID];
     const int tid = threadIdx.x, j = tid & (HID - 1), k = tid / HID;
     const int ldx = (d.in + 3) & ~3;
@@ -174,8 +204,10 @@ __global__ void __launch_bounds__(MT) k_mlp_steps(MlpDims d, const MlpSteps a) {
         const int nparts = (nb + per - 1) / per;
         if ((int)blockIdx.x < nparts) {
             const int s0 = b0 + (int)blockIdx.x * per, s1 = min(b0 + nb, s0 + per);
+            // this CTA's partial, written as it is summed if one sweep makes it
+            double *const part = a.gpart + (size_t)blockIdx.x * d.np;
+            double *const G = a.g_shared && s1 - s0 > MS ? v.g : part;
             mlp_params(d, a.params, s);
-            for (int i = tid; i < d.np; i += MT) G[i] = 0.f;
             double loss = 0.0;
             for (int at = s0; at < s1; at += MS) {
                 const int ns = min(MS, s1 - at);
@@ -192,57 +224,69 @@ __global__ void __launch_bounds__(MT) k_mlp_steps(MlpDims d, const MlpSteps a) {
                         loss += (double)(0.5f * e * e);
                     }
                     s.dy[tid] = e;
+                    v.dy[tid] = e;
                 }
+                for (int i = tid; i < MS * ldx; i += MT) v.x[i] = s.x[i];
+                v.h1[tid] = s.h1[tid];
+                v.h2[tid] = s.h2[tid];
                 __syncthreads();
                 float g2 = 0.f;
                 for (int o = 0; o < d.out; o++) g2 = fmaf(s.w3[o * HID + j], s.dy[k * 8 + o], g2);
                 const float h2 = s.h2[k * HID + j];
-                s.dh2[k * HID + j] = g2 * (1.f - h2 * h2);
+                const float dh2 = g2 * (1.f - h2 * h2);
+                s.dh2[k * HID + j] = dh2;
+                v.dh2[k * HID + j] = dh2;
                 __syncthreads();
                 float g1 = 0.f;
 #pragma unroll 16
                 for (int i = 0; i < HID; i++) g1 = fmaf(s.w2[i * LD2 + j], s.dh2[k * HID + i], g1);
                 const float h1 = s.h1[k * HID + j];
-                s.dh1[k * HID + j] = g1 * (1.f - h1 * h1);
+                v.dh1[k * HID + j] = g1 * (1.f - h1 * h1);
                 __syncthreads();
-                // gradient entries, each one thread's own
-                for (int i = tid; i < HID * HID; i += MT) {
-                    float t = G[d.oW2 + i];
+                // gradient entries, each one thread's own: products and sums in FP64
+                const bool more = at > s0;
+                double hq[MS];
 #pragma unroll
-                    for (int q = 0; q < MS; q++) t = fmaf(s.dh2[q * HID + i / HID], s.h1[q * HID + i % HID], t);
-                    G[d.oW2 + i] = t;
+                for (int q = 0; q < MS; q++) hq[q] = v.h1[q * HID + j];
+#pragma unroll 4
+                for (int r = k; r < HID; r += MS) {
+                    double *const g = G + d.oW2 + r * HID + j;
+                    double t = more ? *g : 0.0;
+#pragma unroll
+                    for (int q = 0; q < MS; q++) t = fma(v.dh2[q * HID + r], hq[q], t);
+                    *g = t;
                 }
                 for (int i = tid; i < HID * d.in; i += MT) {
                     const int r = i / d.in, c = i - r * d.in;
-                    float t = G[d.oW1 + i];
+                    double t = more ? G[d.oW1 + i] : 0.0;
 #pragma unroll
-                    for (int q = 0; q < MS; q++) t = fmaf(s.dh1[q * HID + r], s.x[q * ldx + c], t);
+                    for (int q = 0; q < MS; q++) t = fma(v.dh1[q * HID + r], v.x[q * ldx + c], t);
                     G[d.oW1 + i] = t;
                 }
                 for (int i = tid; i < d.out * HID; i += MT) {
-                    float t = G[d.oW3 + i];
+                    double t = more ? G[d.oW3 + i] : 0.0;
 #pragma unroll
-                    for (int q = 0; q < MS; q++) t = fmaf(s.dy[q * 8 + i / HID], s.h2[q * HID + i % HID], t);
+                    for (int q = 0; q < MS; q++) t = fma(v.dy[q * 8 + i / HID], v.h2[q * HID + i % HID], t);
                     G[d.oW3 + i] = t;
                 }
                 if (tid < HID) {
-                    float t1 = G[d.ob1 + tid], t2 = G[d.ob2 + tid];
+                    double t1 = more ? G[d.ob1 + tid] : 0.0, t2 = more ? G[d.ob2 + tid] : 0.0;
 #pragma unroll
-                    for (int q = 0; q < MS; q++) t1 += s.dh1[q * HID + tid], t2 += s.dh2[q * HID + tid];
+                    for (int q = 0; q < MS; q++) t1 += v.dh1[q * HID + tid], t2 += v.dh2[q * HID + tid];
                     G[d.ob1 + tid] = t1;
                     G[d.ob2 + tid] = t2;
                 }
                 if (tid < d.out) {
-                    float t = G[d.ob3 + tid];
+                    double t = more ? G[d.ob3 + tid] : 0.0;
 #pragma unroll
-                    for (int q = 0; q < MS; q++) t += s.dy[q * 8 + tid];
+                    for (int q = 0; q < MS; q++) t += v.dy[q * 8 + tid];
                     G[d.ob3 + tid] = t;
                 }
             }
-            // (every entry of G was last written by the thread that reads it,
-            // but for the biases and W3 against the strided copy below)
-            __syncthreads();
-            for (int i = tid; i < d.np; i += MT) a.gpart[(size_t)blockIdx.x * d.np + i] = G[i];
+            if (G != part) {
+                __syncthreads();
+                for (int i = tid; i < d.np; i += MT) part[i] = G[i];
+            }
             if (tid < 32) {              // MS * 8 = 32 threads hold the loss
                 loss = warp_sum(loss);
                 if (tid == 0) a.lpart[blockIdx.x] = loss;
@@ -291,7 +335,12 @@ __global__ void __launch_bounds__(MT) k_mlp_steps(MlpDims d, const MlpSteps a) {
 // Host
 // ---------------------------------------------------------------------------
 static size_t fwd_smem(const MlpDims &d) { return mlp_shared_floats(d) * sizeof(float); }
-static size_t steps_smem(const MlpDims &d) { return (mlp_shared_floats(d) + d.np) * sizeof(float); }
+// Training: the FP64 copies, and the gradient of a batch that takes several sweeps
+// if it fits beside them (up to 190 inputs; else it is summed in its partial, in L2).
+constexpr size_t STEPS_SMEM = 220 * 1024;
+static size_t steps_smem(const MlpDims &d, int g_shared) {
+    return mlp_shared_at64(d) + (mlp_shared_doubles(d) + (g_shared ? d.np : 0)) * sizeof(double);
+}
 
 void mlp_create(Mlp &net, int in, int out, uint64_t seed) {
     RP_REQUIRE(in >= 1 && in <= 256 && out >= 1 && out <= 8, -2, "MLP dims: in 1..256, out 1..8");
@@ -325,11 +374,10 @@ void mlp_create(Mlp &net, int in, int out, uint64_t seed) {
     RP_CUDA(cudaMemset(net.m, 0, net.np * sizeof(float)));
     RP_CUDA(cudaMemset(net.v, 0, net.np * sizeof(float)));
     net.step = 0;
-    // for the largest network: a smaller one made later must not lower the limit
-    // of those before it
+    // for any network: a smaller one made later must not lower the limit of those
+    // before it
     const MlpDims most = dims(256, 8);
-    RP_CUDA(cudaFuncSetAttribute(k_mlp_steps, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)steps_smem(most)));
+    RP_CUDA(cudaFuncSetAttribute(k_mlp_steps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STEPS_SMEM));
     RP_CUDA(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)fwd_smem(most)));
 }
@@ -394,20 +442,21 @@ static MlpTrainBuffers mlp_train_buffers(Mlp &net, const float *X_host, const fl
         return r;
     };
     const size_t oX = room((size_t)n * d.in * sizeof(float)), oY = room((size_t)n * d.out * sizeof(float));
-    const size_t oi = room((size_t)n * sizeof(int)), og = room((size_t)b.a.parts * d.np * sizeof(float));
+    const size_t oi = room((size_t)n * sizeof(int)), og = room((size_t)b.a.parts * d.np * sizeof(double));
     const size_t ol = room((size_t)b.nsteps * sizeof(float)), op = room((size_t)b.a.parts * sizeof(double));
     const size_t oc = room(2 * sizeof(unsigned));
     char *p = mlp_room(net, at, st);
     b.a.X = reinterpret_cast<float *>(p + oX);
     b.a.Y = reinterpret_cast<float *>(p + oY);
     b.idx = reinterpret_cast<int *>(p + oi);
-    b.a.gpart = reinterpret_cast<float *>(p + og);
+    b.a.gpart = reinterpret_cast<double *>(p + og);
     b.a.loss = reinterpret_cast<float *>(p + ol);
     b.a.lpart = reinterpret_cast<double *>(p + op);
     b.a.barrier = reinterpret_cast<unsigned *>(p + oc);
     b.a.err = b.a.barrier + 1;
     b.a.n = n;
     b.a.batch = batch;
+    b.a.g_shared = (batch + b.a.parts - 1) / b.a.parts > MS && steps_smem(d, 1) <= STEPS_SMEM;
     b.a.params = net.params;
     b.a.m = net.m;
     b.a.v = net.v;
@@ -423,7 +472,7 @@ static void mlp_steps_launch(Mlp &net, MlpTrainBuffers &b, cudaStream_t st) {
     RP_CUDA(cudaMemsetAsync(b.a.barrier, 0, sizeof(unsigned), st));
     void *args[] = {&d, &b.a};
     RP_CUDA(cudaLaunchCooperativeKernel((const void *)k_mlp_steps, dim3(b.grid), dim3(MT), args,
-                                        steps_smem(d), st));
+                                        steps_smem(d, b.a.g_shared), st));
 }
 
 // The batches' losses (and the error word) after the last launch.
