@@ -3,9 +3,9 @@
 // Adam, FP32.  Parameters are one flat array
 // [W1 (64 x in), b1, W2 (64 x 64), b2, W3 (out x 64), b3], row-major.
 //
-// An epoch of training is one cooperative launch.  Per mini-batch every CTA
-// takes the parameters into shared memory, runs its samples forward and
-// backward four at a time (thread = hidden unit x sample) and writes its
+// An epoch of training is one cooperative launch (of up to 2^16 steps).  Per
+// mini-batch every CTA takes the parameters into shared memory, runs its samples
+// forward and backward four at a time (thread = hidden unit x sample) and writes its
 // gradient partial, products and sums over samples in FP64; after a grid barrier
 // the CTAs share the parameters out, sum the partials in a fixed order and apply
 // Adam (reproducible); after another the next batch starts.  Loss: mean squared
@@ -467,6 +467,10 @@ static MlpTrainBuffers mlp_train_buffers(Mlp &net, const float *X_host, const fl
     return b;
 }
 
+// Steps of one launch: its barrier counts two arrivals of every CTA per step and
+// must not wrap (2^32 is 14 million steps of 148 CTAs; this many take 0.8 s).
+constexpr int MAX_STEPS = 1 << 16;
+
 static void mlp_steps_launch(Mlp &net, MlpTrainBuffers &b, cudaStream_t st) {
     MlpDims d = dims(net.in, net.out);
     RP_CUDA(cudaMemsetAsync(b.a.barrier, 0, sizeof(unsigned), st));
@@ -515,8 +519,15 @@ float mlp_train(Mlp &net, const float *X_host, const float *Y_host, int n, int e
             std::swap(idx[i], idx[k]);
         }
         RP_CUDA(cudaMemcpyAsync(b.idx, idx.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, st));
-        b.a.step0 = net.step;
-        mlp_steps_launch(net, b, st);
+        MlpTrainBuffers part = b;
+        for (int64_t s0 = 0; s0 < b.nsteps; s0 += MAX_STEPS) {
+            const int64_t at = s0 * b.a.batch;
+            part.a.idx = b.a.idx + at;
+            part.a.n = (int)std::min<int64_t>(n - at, (int64_t)MAX_STEPS * b.a.batch);
+            part.a.loss = b.a.loss + s0;
+            part.a.step0 = net.step + (int)s0;
+            mlp_steps_launch(net, part, st);
+        }
         net.step += b.nsteps;
     }
     double tot = 0.0;

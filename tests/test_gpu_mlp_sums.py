@@ -24,3 +24,19 @@ def test_equal_samples_give_one_samples_gradient(cuda, n, n_in, n_out):
     _, many = net.grad(np.repeat(x, n, axis=0), np.repeat(y, n, axis=0))
     assert np.array_equal(many, one)
     net.close()
+
+
+def test_an_epoch_of_more_steps_than_one_launch_takes(cuda):
+    """2^16 + 3 batches of one sample, all equal, so that the shuffle does not
+    matter: the same parameters as 2^16 of them and three more in a second call,
+    and the mean of the losses of both."""
+    rng = np.random.default_rng(5)
+    n, x, y = (1 << 16) + 3, rng.standard_normal((1, 2)).astype(np.float32), np.ones((1, 1), np.float32)
+    nets = [SP.Mlp(2, 1, seed=3), SP.Mlp(2, 1, seed=3)]
+    loss = nets[0].train(np.repeat(x, n, axis=0), np.repeat(y, n, axis=0), epochs=1, batch=1, lr=1e-5)
+    first = nets[1].train(np.repeat(x, n - 3, axis=0), np.repeat(y, n - 3, axis=0), epochs=1, batch=1, lr=1e-5)
+    last = nets[1].train(np.repeat(x, 3, axis=0), np.repeat(y, 3, axis=0), epochs=1, batch=1, lr=1e-5)
+    assert np.array_equal(nets[0].get_params(), nets[1].get_params())
+    assert abs(loss - (first * (n - 3) + last * 3) / n) <= 1e-6 * loss
+    for net in nets:
+        net.close()
