@@ -27,6 +27,8 @@
 
 #include <algorithm>
 #include <cstring>
+#include <map>
+#include <utility>
 
 #include "rp_batch.cuh"
 #include "rp_expm_impl.cuh"
@@ -887,11 +889,9 @@ void batch_free(BatchPlan &bp) {
     if (bp.err) cudaFree(bp.err);
     if (bp.graph) cudaGraphExecDestroy(bp.graph);
     for (auto &q : bp.solo) plan_free(q.plan);
-    for (auto &q : bp.solo_space) {
-        workspace_release(q.second.ws);
-        if (q.second.psi) cudaFree(q.second.psi);
-        if (q.second.tmp) cudaFree(q.second.tmp);
-    }
+    workspace_release(bp.solo_space.ws);
+    if (bp.solo_space.psi) cudaFree(bp.solo_space.psi);
+    if (bp.solo_space.tmp) cudaFree(bp.solo_space.tmp);
     bp = BatchPlan{};
 }
 
@@ -919,7 +919,8 @@ static size_t dyn_smem(const BatchClass &c, int hcap) {
     return 1024 + stage_bytes(c) + table_bytes(c) + (size_t)(2 * hcap + 64) * sizeof(double);
 }
 
-// Team size of a problem given a tile exponent alone: one CTA up to 2^16
+// Team size of a problem given a tile exponent alone, or left to the default where
+// memory is short: one CTA up to 2^16
 // elements, doubling per qubit above, at most 16 (the largest cluster).
 static int default_team(int len) { return std::min(16, 1 << std::max(0, len - 16)); }
 
@@ -969,11 +970,19 @@ static cudaLaunchConfig_t class_config(const BatchClass &c, size_t smem, cudaStr
     return cfg;
 }
 
-void batch_build(BatchPlan &bp, int nprob, const int *len, const int64_t *nterms,
-                 const uint64_t *const *bits, const double *const *coeff, const uint64_t *wbits,
-                 const double *wcoeff, const uint64_t *vbits, const double *vcoeff,
-                 const void *const *psi0, const int *tile, const int *team, int krydim, double tol,
-                 int max_restarts, cudaStream_t st) {
+// The solo problems' space as a workspace of q's size.
+static SoloSpace &solo_space(BatchPlan &bp, const SoloProblem &q) {
+    SoloSpace &sp = bp.solo_space;
+    sp.ws.len = q.len;
+    sp.ws.D = 1ull << q.len;
+    return sp;
+}
+
+static void build_placed(BatchPlan &bp, int nprob, const int *len, const int64_t *nterms,
+                         const uint64_t *const *bits, const double *const *coeff, const uint64_t *wbits,
+                         const double *wcoeff, const uint64_t *vbits, const double *vcoeff,
+                         const void *const *psi0, const int *tile, const int *team, int krydim, double tol,
+                         int max_restarts, bool teams_only, cudaStream_t st) {
     RP_REQUIRE(nprob >= 1, -2, "no problems in the batch");
     RP_REQUIRE(krydim >= 2 && krydim <= BMAXK, -2, "batched krydim must be in [2, 32]");
     RP_REQUIRE(max_restarts >= 1 && max_restarts <= 64, -2, "max_restarts must be in [1, 64]");
@@ -1001,8 +1010,10 @@ void batch_build(BatchPlan &bp, int nprob, const int *len, const int64_t *nterms
         k.second += (double)nterms[p] + (double)(std::unique(xh.begin(), xh.end()) - xh.begin());
     }
     for (const auto &k : kinds)
-        place[k.first] = default_place(k.first, k.second.second / k.second.first, k.second.first,
-                                       1 << std::min(4, std::max(0, k.first - (k.first >= RB ? RB : 8))));
+        place[k.first] = teams_only
+                             ? default_team(k.first)
+                             : default_place(k.first, k.second.second / k.second.first, k.second.first,
+                                             1 << std::min(4, std::max(0, k.first - (k.first >= RB ? RB : 8))));
     for (int p = 0; p < nprob; p++) {
         RP_REQUIRE(len[p] >= 8 && len[p] <= 30, -2, "batched problems need 8..30 qubits");
         RP_REQUIRE(psi0[p] && ((uintptr_t)psi0[p] & 15) == 0, -2, "psi0 must be 16-byte aligned");
@@ -1025,7 +1036,6 @@ void batch_build(BatchPlan &bp, int nprob, const int *len, const int64_t *nterms
             for (uint64_t &b : cut) b &= mask;
             plan_build(q.plan, len[p], 1, cut.data(), coeff[p], nterms[p], default_config(len[p], 1));
             plan_upload(q.plan);
-            bp.solo_space[len[p]];
             continue;
         }
         bp.order.push_back(p);
@@ -1114,14 +1124,17 @@ void batch_build(BatchPlan &bp, int nprob, const int *len, const int64_t *nterms
         }
         c.maxlen = std::max(c.maxlen, probs[p].len);
     }
-    for (auto &q : bp.solo_space) {
-        const size_t vb = sizeof(Cplx<float>) << q.first;
-        if (cudaMalloc(&q.second.psi, vb) != cudaSuccess || cudaMalloc(&q.second.tmp, vb) != cudaSuccess) {
+    if (!bp.solo.empty()) {
+        int most = 0;
+        for (const SoloProblem &q : bp.solo) most = std::max(most, q.len);
+        SoloSpace &sp = bp.solo_space;
+        const size_t vb = sizeof(Cplx<float>) << most;
+        if (cudaMalloc(&sp.psi, vb) != cudaSuccess || cudaMalloc(&sp.tmp, vb) != cudaSuccess) {
             cudaGetLastError();
-            batch_free(bp);
             throw Error{-4, "device out of memory for the batched workspace"};
         }
-        workspace_ensure(q.second.ws, q.first, 1, krydim);
+        workspace_ensure(sp.ws, most, 1, krydim);
+        workspace_matrix(sp.ws, bp.hcap, st);   // for all restarts, as the teams' slots
     }
     if (nb == 0) return;
     RP_CUDA(cudaMalloc((void **)&bp.d_probs, nb * sizeof(BatchProblem)));
@@ -1183,6 +1196,27 @@ void batch_build(BatchPlan &bp, int nprob, const int *len, const int64_t *nterms
     }
     RP_CUDA(cudaMalloc((void **)&bp.err, sizeof(unsigned)));
     RP_CUDA(cudaMemset(bp.err, 0, sizeof(unsigned)));
+}
+
+void batch_build(BatchPlan &bp, int nprob, const int *len, const int64_t *nterms,
+                 const uint64_t *const *bits, const double *const *coeff, const uint64_t *wbits,
+                 const double *wcoeff, const uint64_t *vbits, const double *vcoeff,
+                 const void *const *psi0, const int *tile, const int *team, int krydim, double tol,
+                 int max_restarts, cudaStream_t st) {
+    for (bool teams_only : {false, true}) {
+        try {
+            build_placed(bp, nprob, len, nterms, bits, coeff, wbits, wcoeff, vbits, vcoeff, psi0, tile, team,
+                         krydim, tol, max_restarts, teams_only, st);
+            return;
+        } catch (const Error &e) {
+            batch_free(bp);
+            // the fastest places take more memory than the teams by qubit count do
+            // (a team's slots and the solo problems' space side by side, smaller
+            // teams and so more of them): those next
+            if (teams_only || (e.code != -3 && e.code != -4)) throw;
+            cudaGetLastError();
+        }
+    }
 }
 
 static BatchArgs class_args(const BatchPlan &bp, const BatchClass &c, int ntimes) {
@@ -1249,9 +1283,9 @@ double batch_probe(BatchPlan &bp, int napplies, cudaStream_t st) {
         cudaLaunchConfig_t cfg = class_config(c, c.smem, st, attr);
         RP_CUDA(cudaLaunchKernelEx(&cfg, k_batch_otoc, a));
     }
-    for (auto &q : bp.solo_space) RP_CUDA(cudaMemsetAsync(q.second.ws.err, 0, sizeof(unsigned), st));
+    if (!bp.solo.empty()) RP_CUDA(cudaMemsetAsync(bp.solo_space.ws.err, 0, sizeof(unsigned), st));
     for (SoloProblem &q : bp.solo) {
-        SoloSpace &sp = bp.solo_space[q.len];
+        SoloSpace &sp = solo_space(bp, q);
         RP_CUDA(cudaMemcpyAsync(sp.psi, q.psi0, sizeof(Cplx<float>) << q.len, cudaMemcpyDeviceToDevice, st));
         for (int r = 0; r < napplies; r++) {
             ApplyLaunch L;
@@ -1265,10 +1299,9 @@ double batch_probe(BatchPlan &bp, int napplies, cudaStream_t st) {
     unsigned herr = 0, one = 0;
     if (bp.err) RP_CUDA(cudaMemcpyAsync(&herr, bp.err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     RP_CUDA(cudaStreamSynchronize(st));
-    for (auto &q : bp.solo_space) {
-        RP_CUDA(cudaMemcpy(&one, q.second.ws.err, sizeof(unsigned), cudaMemcpyDeviceToHost));
-        herr |= one;
-    }
+    if (!bp.solo.empty())
+        RP_CUDA(cudaMemcpy(&one, bp.solo_space.ws.err, sizeof(unsigned), cudaMemcpyDeviceToHost));
+    herr |= one;
     float ms = 0.f;
     RP_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     cudaEventDestroy(e0);
@@ -1360,7 +1393,7 @@ __global__ void k_string(uint32_t x, uint32_t z, float cr, float ci, const Cplx<
 
 // One OTOC point of a solo problem, as team_otoc; returns its H.psi count.
 static int solo_otoc(BatchPlan &bp, SoloProblem &q, double t, double *f, cudaStream_t st) {
-    SoloSpace &sp = bp.solo_space[q.len];
+    SoloSpace &sp = solo_space(bp, q);
     const uint32_t n = 1u << q.len;
     const int grid = (int)std::min<uint32_t>((n + 255) / 256, 8u * (uint32_t)num_sms());
     auto string = [&](bool w, const void *in, void *out) {

@@ -2,7 +2,6 @@
 // problems, uneven qubit counts, one persistent launch per time step.
 #pragma once
 
-#include <map>
 #include <vector>
 
 #include "rp_apply.cuh"
@@ -44,7 +43,8 @@ struct SoloProblem {
     float wcr = 0, wci = 0, vcr = 0, vci = 0;
 };
 
-// What the solo problems of one qubit count share.
+// What the solo problems share: they run one after the other, so vectors of the
+// largest one's size serve them all.
 struct SoloSpace {
     KryWorkspace ws;
     void *psi = nullptr, *tmp = nullptr;
@@ -69,7 +69,7 @@ struct BatchPlan {
     cudaGraphExec_t graph = nullptr;
     std::vector<double> graph_times;
     std::vector<SoloProblem> solo;
-    std::map<int, SoloSpace> solo_space;     // by qubit count
+    SoloSpace solo_space;
 };
 
 // Problem p: len[p] qubits, nterms[p] terms (bits, coeff as for rp_ham_create),
@@ -79,7 +79,7 @@ struct BatchPlan {
 // Tile 12 selects the row-tile loop (2-D TMA, 4096-element swizzled tiles)
 // for states of at least 2^12 elements.  A problem with neither given goes where
 // its size and the number of its kind put it: into a team, or alone on the whole
-// GPU (solo).
+// GPU (solo); where memory is too short for that, into a team of default_team CTAs.
 void batch_build(BatchPlan &bp, int nprob, const int *len, const int64_t *nterms,
                  const uint64_t *const *bits, const double *const *coeff, const uint64_t *wbits,
                  const double *wcoeff, const uint64_t *vbits, const double *vcoeff,

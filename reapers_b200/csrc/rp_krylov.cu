@@ -45,7 +45,7 @@ static bool fused_projections() {
     return v == 1;
 }
 
-static void grow_hfull(KryWorkspace &ws, int need, cudaStream_t st) {
+void workspace_matrix(KryWorkspace &ws, int need, cudaStream_t st) {
     if (need <= ws.hcap) return;
     int cap = std::max(ws.hcap ? ws.hcap : 4 * ws.krydim, 32);
     while (cap < need) cap *= 2;
@@ -334,7 +334,7 @@ void krylov_evolve(const ApplyPlan &plan, KryWorkspace &ws, void *psi, double t_
     KryDev const *hdr = nullptr;
     while (true) {
         cycle++;
-        grow_hfull(ws, cycle * krydim, st);
+        workspace_matrix(ws, cycle * krydim, st);
         arnoldi_cycle(plan, ws, krydim, cycle > 1, st);
         VecTable tab{};
         for (int i = 0; i <= krydim; i++) tab.p[i] = ws.u[i];

@@ -58,6 +58,9 @@ struct KryWorkspace {
 // a workspace for the same state shape is kept and grown, never shrunk
 // (rp_workspace_release frees it).
 void workspace_ensure(KryWorkspace &ws, int len, int dtype, int krydim);
+// Room for a block Hessenberg matrix of `need` rows and its exponential (an evolve
+// makes it cycle by cycle where it is not there yet).
+void workspace_matrix(KryWorkspace &ws, int need, cudaStream_t st);
 void workspace_release(KryWorkspace &ws);
 // The pinned host copy of a KryDev that the calls read their results through, and
 // the Lanczos steps' device state.
