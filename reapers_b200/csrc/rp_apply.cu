@@ -53,6 +53,30 @@ constexpr int ROW_MERGE_MIN_LEN = 22;
 constexpr int SPLIT_MIN_LEN = 17;
 constexpr size_t SPLIT_MIN_RUNS = 64;
 
+// Lists too long for the row kernel's table: the run kernel, unless the terms
+// hardly share their X masks.  The tiled kernel takes a term in the same time
+// whatever its mask (one with both a real and an imaginary coefficient takes 1.17
+// times as long); the run kernel pays mostly for the masks it gathers, once more
+// for a mask with coefficients of both kinds, and little for a term.  Random strings,
+// ms (run / tiled): 2^22 complex64, 6000 terms, of 100 % distinct masks 19.3 / 16.5, 90 %
+// 17.8 / 16.5, 80 % 16.1 / 16.5, 70 % 14.5 / 16.5; complex128 22.0 / 21.2, 20.3 / 21.1;
+// with complex coefficients, 100 % 28.2 / 19.5 and 33.2 / 24.0; 2^26 complex64, 2200 terms
+// 149 / 127.  Dense SYK, 2^22, 18 terms per mask 94 / 375.  Up to 2^19 elements the run
+// kernel is taken as it is: 2^18 complex64, 3000 masks 0.65 / 1.5, 2^19 1.02 / 1.13 (2500
+// terms; with complex coefficients 1.50 / 1.26, of 6000 terms 3.5 / 3.6).
+constexpr int RUNS_ALWAYS_LEN = 19;
+constexpr double RUNS_MASK = 0.6, RUNS_KIND = 0.31, RUNS_TERM = 0.2;   // of a tiled term's time
+constexpr double TILED_TERM_C64 = 1.0, TILED_TERM_C128 = 1.06, TILED_EXTRA = 0.17;
+
+static bool scattered(const RunPlan &p, int dtype, int64_t nterms) {
+    double kinds = 0.0;
+    for (const Run &r : p.runs) kinds += (r.nr > 0) + (r.ni > 0);
+    const double records = (double)p.terms.size();
+    const double runs = RUNS_MASK * (double)p.runs.size() + RUNS_KIND * kinds + RUNS_TERM * records;
+    return runs > (dtype == 2 ? TILED_TERM_C128 : TILED_TERM_C64) * (double)nterms +
+                      TILED_EXTRA * (records - (double)nterms);
+}
+
 static size_t elem_size(int dtype) { return dtype == 2 ? 16 : 8; }
 
 ApplyConfig default_config(int len, int dtype) {
@@ -183,6 +207,12 @@ void plan_build(ApplyPlan &plan, int len, int dtype, const uint64_t *bits,
         return;
     }
     runplan_build(plan.runs, len, bits, coeff, nterms);
+    if (len > RUNS_ALWAYS_LEN && scattered(plan.runs, dtype, nterms)) {
+        plan.runs = RunPlan{};
+        if (dtype == 2) build_terms<double>(plan, bits, coeff, nterms);
+        else build_terms<float>(plan, bits, coeff, nterms);
+        return;
+    }
     if (len < SPLIT_MIN_LEN || plan.runs.runs.size() < SPLIT_MIN_RUNS) return;
     splitplan_build(plan.split, len, dtype, bits, coeff, nterms);
     if (plan.split.ok) plan.runs = RunPlan{};
