@@ -194,13 +194,13 @@ def ground_state(ham, krydim=5, eps=None, maxiter=0, seed=0):
     if eps is None:
         eps = 10 * float(np.finfo(prec).eps)
     v0 = random_state(ham.len, "c64" if ham.dtype == RP_C64 else "c128", seed=seed)
-    vecs = None
+    room = None
     numiter = 0
     while True:
         if m <= 64:   # what rp_lanczos takes
-            if vecs is None:
-                vecs = [torch.empty_like(v0) for _ in range(m)]
-            alpha, beta, ritz = _lanczos(ham, v0, m, vecs)
+            if room is None:
+                room = _lanczos_room(v0, m)
+            alpha, beta, ritz = _lanczos(ham, v0, m, room)
         else:
             alpha, beta, ritz = _lanczos_calls(ham, v0, m)
         evals, evecs = eigh_tridiagonal(np.array(alpha), np.array(beta[:len(alpha) - 1]))
@@ -208,21 +208,27 @@ def ground_state(ham, krydim=5, eps=None, maxiter=0, seed=0):
         g = ritz(evecs[:, idx])
         scale(g, 1.0 / norm(g))
         numiter += 1
-        if vecs is not None:   # the Ritz vector took the last one's place
-            vecs = [v0] + vecs[:-1]
+        if room is not None:   # the Ritz vector took the last one's place
+            room = (room[0], v0)
         v0 = g
         if not (beta and beta[0] > eps and (not maxiter or numiter < maxiter)):
             return float(evals[idx]), g
 
 
-def _lanczos(ham, v0, m, vecs=None):
-    """m Lanczos steps from v0 in one call, into the m vectors `vecs`: (alpha,
-    beta, function giving the basis' combination with real coefficients, in the
-    last of them)."""
+def _lanczos_room(v0, m):
+    """The m vectors that _lanczos writes beside v0: all but the last as one tensor."""
     import torch
-    if vecs is None:
-        vecs = [torch.empty_like(v0) for _ in range(m)]
-    ptrs = (C.c_void_p * (m + 1))(*[_ptr(t).value for t in [v0] + vecs])
+    return (torch.empty((m - 1, v0.numel()), dtype=v0.dtype, device=v0.device), torch.empty_like(v0))
+
+
+def _lanczos(ham, v0, m, room=None):
+    """m Lanczos steps from v0 in one call, into `room`: (alpha, beta, function
+    giving the basis' combination with real coefficients, in the last vector of
+    the room)."""
+    basis, last = _lanczos_room(v0, m) if room is None else room
+    vecs = (v0, basis, last)   # (the function returned keeps them alive)
+    at, step = basis.data_ptr(), basis.stride(0) * basis.element_size()
+    ptrs = (C.c_void_p * (m + 1))(_ptr(v0).value, *range(at, at + (m - 1) * step, step), _ptr(last).value)
     alpha, beta, k = (C.c_double * m)(), (C.c_double * m)(), C.c_int()
     _lib.call("rp_lanczos", ham.handle, ptrs, m, alpha, beta, C.byref(k))
 
