@@ -36,10 +36,10 @@ static constexpr int stages_for(int B) {
     return s < 2 ? 2 : (s > 8 ? 8 : s);
 }
 
-// Row plans with a fused diagonal from this size on are merged (coefficients of
-// a row summed before they are applied).  Smaller states keep the order of
-// single terms, and with it their last bits, on which the step controller's
-// decisions hang.
+// Row plans with a fused diagonal may be merged (coefficients of a row summed
+// before they are applied) from this size on.  Below it the plans keep the order of
+// single terms; the line was not drawn by time (XXZ chain, us, plain / merged: 2^20
+// complex64 21.1 / 19.8, complex128 39.4 / 35.2).
 constexpr int ROW_MERGE_MIN_LEN = 22;
 
 // States below the row kernel's size: the run kernel, which reads a vector per

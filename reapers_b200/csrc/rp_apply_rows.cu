@@ -34,8 +34,8 @@
 // output's own tile) every row sums their coefficients, signed by its high
 // index bits, into one bucket per in-row Z pattern, and a Walsh-Hadamard
 // transform over the in-row bits gives each element's diagonal factor,
-// applied once to the own row.  Merged plans (MODE 2, from 2^22 elements on) are
-// bound by instruction issue, not by their bytes, so they spare instructions:
+// applied once to the own row.  Merged plans (MODE 2, from 2^22 elements on, where
+// merge_pays) are bound by instruction issue, not by their bytes, so they spare instructions:
 // terms of an X mask with equal chunk signs (a bond's XX and YY) are summed to
 // one coefficient per row first, a record says whether the next one belongs to
 // it, and the part of the diagonal without a Z bit in the tile is summed over the
@@ -109,6 +109,24 @@ static void row_mark_next(std::vector<RowTerm<float>> &terms, size_t first, size
         if (!(terms[k + 1].cs & ROW_SAME_SRC)) continue;
         terms[k].cs |= ROW_NEXT_SAME | (terms[k + 1].js == terms[k].js ? ROW_NEXT_MERGE : 0u);
     }
+}
+
+// Whether a merged plan is the faster one, by what it spares against what it costs:
+// a term summed into the one before it is worth four terms of the diagonal taken
+// once per tile; the sum over the lanes costs every tile the same, the look-ahead
+// every term that stays (complex64 has twice the elements per row, so the diagonal
+// terms are worth half as much to it).  us, plain / merged, at 2^24 elements
+// (complex64; complex128): XXZ chain 308 / 286; 625 / 550, XX + YY of all pairs
+// 2444 / 2108; 5247 / 4457, ZZ of all pairs and X fields 336 / 322; 730 / 669, transverse
+// Ising chain (12 folded) 251 / 255; 494 / 483, 100 and 16 folded Z strings alone 86 / 74
+// and 64 / 72; 175 / 121 and 119 / 118, random Z strings 65 / 78 (4), 145 / 157 (200); 118 /
+// 154 (16), 276 / 285, half of 200 random strings diagonal 1030 / 1090; 2269 / 2536.
+static bool merge_pays(const RowPlan &rp, int dtype) {
+    int summed = 0;
+    for (const RowTerm<float> &t : rp.terms) summed += (t.cs & ROW_NEXT_MERGE) != 0;
+    const int rest = rp.nterms - summed;
+    const int cost = dtype == 2 ? (rest ? 8 : 20) : (rest ? 30 + rest / 2 : 50);
+    return 4 * summed + rp.nfold > cost;
 }
 
 // CTAs per SM (RPB200_ROW_CTAS, 1 or 2; default 2): the shared memory of an SM
@@ -230,6 +248,10 @@ void rowplan_build(RowPlan &rp, int len, int dtype, const uint64_t *bits, const 
     rp.B = B;
     rp.ntiles = 1 << (len - B);
     rp.nterms = (int)rp.terms.size();
+    if (rp.merged && !merge_pays(rp, dtype)) {
+        rowplan_build(rp, len, dtype, bits, coeff, nterms, any_len, fuse_diag, false);
+        return;
+    }
     // CTAs in flight: two per SM by default (measured fastest on B200:
     // 47.7 ms vs 67.3 ms with one per SM and 77.6 ms with an aligned
     // 128-CTA window at N = 56); RPB200_ROW_GRID overrides it for tuning.

@@ -81,7 +81,7 @@ constexpr uint32_t ROW_NEXT_SAME = 1u << 15, ROW_NEXT_MERGE = 1u << 16;
 // kernel); otherwise only for states of at least 128 tiles.  fuse_diag: fold
 // the real Z strings into the per-row diagonal factor (single-state kernel).
 // merged: with it, order the terms for coefficients summed per row and fold the
-// tile's part of the diagonal.
+// tile's part of the diagonal, where that is faster.
 void rowplan_build(RowPlan &rp, int len, int dtype, const uint64_t *bits, const double *coeff,
                    int64_t nterms, bool any_len = false, bool fuse_diag = false, bool merged = false);
 void rowplan_upload(RowPlan &rp);
