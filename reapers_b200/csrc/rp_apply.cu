@@ -49,9 +49,16 @@ constexpr int ROW_MERGE_MIN_LEN = 22;
 // 18.6, 2^17 35.0 / 21.2, 2^18 56 / 33; 2^16 complex128 20.7 / 21.4, 2^17 39 /
 // 33.  With few runs the split kernel's tile loads do not pay: XXZ chain (17
 // runs) 2^17 8.5 / 13.4, 2^18 12.5 / 14.5; 60 random strings 12.7 / 13.3 and
-// 19.6 / 17.5.
+// 19.6 / 17.5.  The run kernel gives a block of outputs eight warps whatever its
+// runs, the tiled kernel a thread per element: a single string 2^17 3.23 / 2.67 (run /
+// tiled; two 3.33 / 3.27, in complex128 3.80 / 3.32), 2^18 5.53 / 2.90, four 5.85 / 4.75,
+// eight 6.44 / 7.27.
 constexpr int SPLIT_MIN_LEN = 17;
 constexpr size_t SPLIT_MIN_RUNS = 64;
+
+static bool few_terms(int len, int dtype, int64_t nterms) {
+    return len >= SPLIT_MIN_LEN && nterms <= (len > 17 ? 6 : dtype == 2 ? 2 : 1);
+}
 
 // Lists too long for the row kernel's table: the run kernel, unless the terms
 // hardly share their X masks.  The tiled kernel takes a term in the same time
@@ -206,8 +213,9 @@ void plan_build(ApplyPlan &plan, int len, int dtype, const uint64_t *bits,
         plan.alg_bytes = plan.rows.alg_bytes_smem;
         return;
     }
-    runplan_build(plan.runs, len, bits, coeff, nterms);
-    if (len > RUNS_ALWAYS_LEN && scattered(plan.runs, dtype, nterms)) {
+    const bool few = few_terms(len, dtype, nterms);
+    if (!few) runplan_build(plan.runs, len, bits, coeff, nterms);
+    if (few || (len > RUNS_ALWAYS_LEN && scattered(plan.runs, dtype, nterms))) {
         plan.runs = RunPlan{};
         if (dtype == 2) build_terms<double>(plan, bits, coeff, nterms);
         else build_terms<float>(plan, bits, coeff, nterms);
