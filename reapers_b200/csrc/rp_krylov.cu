@@ -452,7 +452,8 @@ void krylov_combine(KryWorkspace &ws, const ArnoldiResult &R, const double *coef
 // just written, past L1.  The sums are the same, bit for bit.  Measured, four
 // factors, one call of rp_expm_first_columns with its copies, scratch and 256
 // threads -> this: m = 16 99 -> 100 us, m = 31 250 -> 191, m = 37 321 -> 244, and by
-// the threads alone m = 38 330 -> 270, m = 65 1024 -> 741.
+// the threads alone m = 38 330 -> 270, m = 65 1024 -> 741.  Below m = 11 the barriers of
+// 512 threads cost more than they bring (m = 4 58 us, with 256 50).
 constexpr size_t CANDS_SMEM = 224 * 1024;
 __global__ void __launch_bounds__(512) k_expm_cands(int m, const cd *H, const double *fr, const double *fi,
                                                     cd *scratch, cd *col0, int in_smem) {
@@ -488,7 +489,7 @@ void expm_candidates(int m, const double *H, int ncand, const double *fr, const 
     const size_t smem = in_smem ? all : fac;
     // the same value on every call: calls of other sizes, threads and devices cannot lower it
     RP_CUDA(cudaFuncSetAttribute(k_expm_cands, cudaFuncAttributeMaxDynamicSharedMemorySize, CANDS_SMEM));
-    k_expm_cands<<<ncand, 512, smem, st>>>(m, dH, dfr, dfi, scr, dcol, in_smem);
+    k_expm_cands<<<ncand, m <= 10 ? 256 : 512, smem, st>>>(m, dH, dfr, dfi, scr, dcol, in_smem);
     RP_CUDA(cudaGetLastError());
     RP_CUDA(cudaMemcpyAsync(col0, dcol, (size_t)ncand * m * sizeof(cd), cudaMemcpyDeviceToHost, st));
     RP_CUDA(cudaStreamSynchronize(st));

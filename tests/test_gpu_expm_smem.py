@@ -35,3 +35,21 @@ def test_every_size_launches(cuda, m, cycles):
     r = subprocess.run([sys.executable, "-c", CODE.format(m=m, cycles=cycles)], cwd=ROOT, capture_output=True,
                        text=True, timeout=300)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("n", [9, 10, 11])
+def test_first_columns_around_the_change_of_threads(cuda, n):
+    """Ten rows are the last for a CTA of 256 threads; 1e-13 as for the other sizes
+    without squarings (|f A| stays below 5.37 in the 1-norm)."""
+    import numpy as np
+    import scipy.linalg as sla
+
+    import reapers_b200 as rb
+    from reapers_b200 import stepper as SP
+    rb.init(0)
+    rng = np.random.default_rng(n)
+    A = rng.standard_normal((n, n)) + 1j * rng.standard_normal((n, n))
+    A *= 4.0 / np.abs(A).sum(axis=0).max()
+    f = np.exp(2j * np.pi * np.arange(4) / 4) * np.linspace(1.3, 0.01, 4)
+    ref = np.stack([sla.expm(v * A)[:, 0] for v in f])
+    assert np.max(np.abs(SP.expm_first_columns(A, f) - ref)) <= 1e-13 * max(1.0, np.max(np.abs(ref)))
