@@ -196,31 +196,30 @@ void plan_build(ApplyPlan &plan, int len, int dtype, const uint64_t *bits,
     plan.rows = RowPlan{};
     plan.split = SplitPlan{};
     plan.runs = RunPlan{};
-    if (cfg.tiled || nterms == 0) {
+    auto tiled = [&] {
         if (dtype == 2) build_terms<double>(plan, bits, coeff, nterms);
         else build_terms<float>(plan, bits, coeff, nterms);
         plan.ngroups = (int)plan.groups.size();
-    } else {   // the tiled kernel's group count, for the plan's figures
-        std::vector<uint32_t> xh(nterms);
-        for (int64_t k = 0; k < nterms; k++) xh[k] = even_bits(bits[k]) >> cfg.B;
-        std::sort(xh.begin(), xh.end());
-        plan.ngroups = (int)(std::unique(xh.begin(), xh.end()) - xh.begin());
-    }
-    plan.alg_bytes = (double)(plan.ngroups + 1) * D * (double)elem_size(dtype);
-    if (cfg.tiled || nterms == 0) return;
+        plan.alg_bytes = (double)(plan.ngroups + 1) * D * (double)elem_size(dtype);
+    };
+    if (cfg.tiled || nterms == 0) return tiled();
     rowplan_build(plan.rows, len, dtype, bits, coeff, nterms, false, true, len >= ROW_MERGE_MIN_LEN);
     if (plan.rows.ok) {
+        plan.ngroups = (int)plan.rows.groups.size();
         plan.alg_bytes = plan.rows.alg_bytes_smem;
         return;
     }
-    const bool few = few_terms(len, dtype, nterms);
-    if (!few) runplan_build(plan.runs, len, bits, coeff, nterms);
-    if (few || (len > RUNS_ALWAYS_LEN && scattered(plan.runs, dtype, nterms))) {
+    if (few_terms(len, dtype, nterms)) return tiled();
+    runplan_build(plan.runs, len, bits, coeff, nterms);
+    if (len > RUNS_ALWAYS_LEN && scattered(plan.runs, dtype, nterms)) {
         plan.runs = RunPlan{};
-        if (dtype == 2) build_terms<double>(plan, bits, coeff, nterms);
-        else build_terms<float>(plan, bits, coeff, nterms);
-        return;
+        return tiled();
     }
+    // the tiled kernel's group count, for the plan's figures (runs are sorted by mask)
+    plan.ngroups = 0;
+    for (size_t r = 0; r < plan.runs.runs.size(); r++)
+        plan.ngroups += r == 0 || plan.runs.runs[r].x >> cfg.B != plan.runs.runs[r - 1].x >> cfg.B;
+    plan.alg_bytes = (double)(plan.ngroups + 1) * D * (double)elem_size(dtype);
     if (len < SPLIT_MIN_LEN || plan.runs.runs.size() < SPLIT_MIN_RUNS) return;
     splitplan_build(plan.split, len, dtype, bits, coeff, nterms);
     if (plan.split.ok) plan.runs = RunPlan{};

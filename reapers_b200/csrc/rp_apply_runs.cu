@@ -268,10 +268,18 @@ void runplan_build(RunPlan &p, int len, const uint64_t *bits, const double *coef
         if (cr != 0.0 || ci == 0.0) ts.push_back({x, z, s * cr, 0});
         if (ci != 0.0) ts.push_back({x, z, s * ci, 1});
     }
+    // by mask, then kind of coefficient, in the list's order among equals: a byte of
+    // the key at a time, least significant first
+    std::vector<T> other(ts.size());
+    for (int shift = 0; shift <= len; shift += 8) {
+        auto digit = [shift](const T &t) { return (((uint64_t)t.x << 1 | (uint64_t)t.kind) >> shift) & 255u; };
+        size_t at[257] = {};
+        for (const T &t : ts) at[digit(t) + 1]++;
+        for (int d = 0; d < 256; d++) at[d + 1] += at[d];
+        for (const T &t : ts) other[at[digit(t)]++] = t;
+        ts.swap(other);
+    }
     p.eb = std::min(3, len - 5);
-    std::stable_sort(ts.begin(), ts.end(), [](const T &a, const T &b) {
-        return a.x != b.x ? a.x < b.x : a.kind < b.kind;
-    });
     double total = 0.0;
     for (size_t k = 0; k < ts.size(); k++)
         total += TERM_COST + (k == 0 || ts[k].x != ts[k - 1].x ? RUN_COST : 0.0);
@@ -281,6 +289,7 @@ void runplan_build(RunPlan &p, int len, const uint64_t *bits, const double *coef
     p.parts = std::min({MAX_PARTS, 2 * num_sms() / p.nblocks, (int)(total / (MIN_SHARE * RUN_W))});
     p.parts = std::max(p.parts, 1);
     const int workers = p.parts * RUN_W;
+    p.terms.reserve(ts.size());
     // contiguous shares of equal cost; a run cut by a boundary continues as
     // another run of the next worker
     p.wstart.assign(1, 0u);
