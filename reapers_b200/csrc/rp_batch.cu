@@ -891,7 +891,6 @@ void batch_free(BatchPlan &bp) {
     for (auto &q : bp.solo) plan_free(q.plan);
     workspace_release(bp.solo_space.ws);
     if (bp.solo_space.psi) cudaFree(bp.solo_space.psi);
-    if (bp.solo_space.tmp) cudaFree(bp.solo_space.tmp);
     bp = BatchPlan{};
 }
 
@@ -1129,10 +1128,11 @@ static void build_placed(BatchPlan &bp, int nprob, const int *len, const int64_t
         for (const SoloProblem &q : bp.solo) most = std::max(most, q.len);
         SoloSpace &sp = bp.solo_space;
         const size_t vb = sizeof(Cplx<float>) << most;
-        if (cudaMalloc(&sp.psi, vb) != cudaSuccess || cudaMalloc(&sp.tmp, vb) != cudaSuccess) {
+        if (cudaMalloc(&sp.psi, 2 * vb) != cudaSuccess) {
             cudaGetLastError();
             throw Error{-4, "device out of memory for the batched workspace"};
         }
+        sp.tmp = static_cast<char *>(sp.psi) + vb;
         workspace_ensure(sp.ws, most, 1, krydim);
         workspace_matrix(sp.ws, bp.hcap, st);   // for all restarts, as the teams' slots
     }

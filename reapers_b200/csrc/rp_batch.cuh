@@ -47,7 +47,7 @@ struct SoloProblem {
 // largest one's size serve them all.
 struct SoloSpace {
     KryWorkspace ws;
-    void *psi = nullptr, *tmp = nullptr;
+    void *psi = nullptr, *tmp = nullptr;     // one allocation
 };
 
 struct BatchPlan {

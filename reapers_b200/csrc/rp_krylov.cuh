@@ -42,6 +42,7 @@ struct EvolveStats {
 struct KryWorkspace {
     int len = 0, dtype = 0, krydim = 0;
     uint64_t D = 0;
+    std::vector<void *> mem;   // allocations of the vectors and of all but hfull, escratch
     std::vector<void *> u;
     void *y = nullptr;
     KryDev *dev = nullptr;
