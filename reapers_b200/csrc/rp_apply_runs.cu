@@ -51,6 +51,7 @@ struct RunArgs {
     Cplx<Real> *partial;                 // [part][element]
     unsigned *arrived;                   // per block, 0 between launches
     int parts;
+    int span;                            // planned workers' shares that a warp takes
     size_t dim;
     double alpha;
     const double *alpha_dev;
@@ -103,8 +104,8 @@ __global__ void __launch_bounds__(RUN_T, 2) k_apply_runs(const RunArgs<Real> a) 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned rank = blockIdx.x % (unsigned)a.parts;
     const uint32_t block = blockIdx.x / (unsigned)a.parts;
-    const int worker = (int)rank * RUN_W + warp;
-    const uint32_t r1 = a.wstart[worker + 1];
+    const int worker = ((int)rank * RUN_W + warp) * a.span;
+    const uint32_t r1 = a.wstart[worker + a.span];
     uint32_t r = a.wstart[worker];
     Cplx<Real> acc[E];
 #pragma unroll
@@ -340,13 +341,21 @@ static void launch_runs(const RunPlan &p, const RunLaunch &l, cudaStream_t st) {
     a.wstart = reinterpret_cast<const uint32_t *>(p.dev + p.at_wstart);
     a.partial = reinterpret_cast<Cplx<Real> *>(p.dev + p.at_partial);
     a.arrived = reinterpret_cast<unsigned *>(p.dev + p.at_arrived);
-    a.parts = p.parts;
+    // Captured products keep nothing with the plan: replays of two graphs may overlap,
+    // on other streams than the library's, and would share the partial sums.  One CTA
+    // then takes all parts of its block, us outside / inside a graph / tiled kernel there:
+    // sparse SYK, complex128, 12 qubits 6.1 / 10.2 / 49, 14 qubits 7.5 / 11.7 / 86; dense SYK,
+    // 8 qubits 6.6 / 29 / 377, 12 qubits 16.7 / 117 / 2283.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (p.parts > 1) RP_CUDA(cudaStreamIsCapturing(st, &capture));
+    a.span = capture == cudaStreamCaptureStatusNone ? 1 : p.parts;
+    a.parts = p.parts / a.span;
     a.dim = (size_t)p.nblocks * (32u << EB);
     a.alpha = l.alpha;
     a.alpha_dev = l.alpha_dev;
     a.accumulate = l.accumulate;
     a.active = l.active;
-    launch_dependent(k_apply_runs<Real, EB>, p.nblocks * p.parts, RUN_T, 0, st, 1, a);
+    launch_dependent(k_apply_runs<Real, EB>, p.nblocks * a.parts, RUN_T, 0, st, 1, a);
 }
 
 template <typename Real>

@@ -56,8 +56,8 @@ struct RunPlan {
     std::vector<Run> runs;               // cut at the workers' boundaries
     std::vector<uint32_t> wstart;        // worker -> first run (workers + 1 entries)
     // one allocation: terms, runs, wstart, and (parts > 1) the parts' partial
-    // sums and the blocks' arrival counts; a plan's launches run one after the
-    // other (all on the library's stream)
+    // sums and the blocks' arrival counts, for the launches on the library's stream,
+    // which run one after the other (captured ones do without: launch_runs)
     char *dev = nullptr;
     size_t at_runs = 0, at_wstart = 0, at_arrived = 0, at_partial = 0;
 };
