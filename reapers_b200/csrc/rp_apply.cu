@@ -234,7 +234,7 @@ void plan_upload(ApplyPlan &plan) {
     if (plan.rows.ok || plan.split.ok || plan.runs.ok) {
         rowplan_upload(plan.rows);
         splitplan_upload(plan.split);
-        runplan_upload(plan.runs, plan.len, plan.dtype);
+        runplan_upload(plan.runs);
         return;
     }
     size_t tb = plan.term_bytes.size();

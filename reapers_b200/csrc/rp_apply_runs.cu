@@ -2,16 +2,17 @@
 // coefficients of the terms with X mask x, signed by (-1)^popc(z & n).
 //
 // Used below the row kernel's size, and above it for lists too long for that
-// kernel's table whose terms share X masks (plan_build has the rules).  For states up
-// to 2^14 elements a term's cost is its instructions, not its bytes (the state
-// sits in L1 / L2), and there are too few tiles of output to fill the GPU.  So the work is cut both ways: a warp owns 32 << eb output
-// elements (lane = the low 5 index bits, eb bits in registers) and one worker's
-// share of the terms; the eight warps of `parts` CTAs are the workers of one
-// block of outputs.  Their sums meet in shared memory and then in the plan's
-// partial buffer, where the block's last CTA to arrive adds the parts in order
-// (one launch, and the same bits run to run).  Clusters in place of the buffer
-// were slower: eight-CTA clusters left 55 of 148 SMs idle while others held
-// two CTAs (dense SYK on 12 qubits 28 us, against the figures below).
+// kernel's table whose terms share X masks (plan_build has the rules).  For states
+// up to 2^14 elements a term's cost is its instructions, not its bytes (the state
+// sits in L1 / L2), and there are too few tiles of output to fill the GPU.  So the
+// work is cut both ways: a warp owns 32 << eb output elements (lane = the low 5
+// index bits, eb bits in registers) and one worker's share of the terms; the eight
+// warps of `parts` CTAs are the workers of one block of outputs.  Their sums meet in
+// shared memory and then in a buffer of partial sums, where the block's last CTA to
+// arrive adds the parts in order (one launch, and the same bits run to run).
+// Clusters in place of the buffer were slower: eight-CTA clusters left 55 of 148 SMs
+// idle while others held two CTAs (dense SYK on 12 qubits 28 us, against the figures
+// below).
 //
 // Terms with one X mask form a run: the run's diagonal factor is summed first
 // and then multiplied once with the gathered elements, so the loads and
@@ -314,16 +315,38 @@ void runplan_build(RunPlan &p, int len, const uint64_t *bits, const double *coef
     p.ok = true;
 }
 
-void runplan_upload(RunPlan &p, int len, int dtype) {
+// Partial sums and arrival counts of blocks that several CTAs share: one buffer for
+// all plans, whose launches run one after the other on the library's stream (captured
+// ones do without it).  Shared blocks have at most two CTAs per SM in all, so its size
+// is fixed; a buffer per plan cost 0.37 ms of a plan's creation.
+static char *g_runs = nullptr;
+
+static size_t runs_partial_bytes() { return (size_t)2 * num_sms() * 256 * sizeof(Cplx<double>); }
+
+static char *runs_scratch() {
+    if (g_runs) return g_runs;
+    const size_t count = (size_t)2 * num_sms() * sizeof(unsigned);
+    void *p = nullptr;
+    RP_CUDA(cudaMalloc(&p, runs_partial_bytes() + count));
+    g_runs = static_cast<char *>(p);
+    RP_CUDA(cudaMemset(g_runs + runs_partial_bytes(), 0, count));
+    return g_runs;
+}
+
+void runs_scratch_release() {
+    if (g_runs) cudaFree(g_runs);
+    g_runs = nullptr;
+}
+
+void runplan_upload(RunPlan &p) {
     if (!p.ok) return;
     runplan_free(p);
     TablePack t;
     t.add(p.terms);
     p.at_runs = t.add(p.runs);
     p.at_wstart = t.add(p.wstart);
-    p.at_arrived = t.room(p.nblocks * sizeof(unsigned));
-    p.at_partial = t.bytes.size();
-    p.dev = t.upload(p.parts > 1 ? ((size_t)p.parts << len) * (dtype == 2 ? 16 : 8) : 0);
+    p.dev = t.upload();
+    if (p.parts > 1) runs_scratch();
 }
 
 void runplan_free(RunPlan &p) {
@@ -339,10 +362,8 @@ static void launch_runs(const RunPlan &p, const RunLaunch &l, cudaStream_t st) {
     a.terms = reinterpret_cast<const RunTerm *>(p.dev);
     a.runs = reinterpret_cast<const Run *>(p.dev + p.at_runs);
     a.wstart = reinterpret_cast<const uint32_t *>(p.dev + p.at_wstart);
-    a.partial = reinterpret_cast<Cplx<Real> *>(p.dev + p.at_partial);
-    a.arrived = reinterpret_cast<unsigned *>(p.dev + p.at_arrived);
-    // Captured products keep nothing with the plan: replays of two graphs may overlap,
-    // on other streams than the library's, and would share the partial sums.  One CTA
+    // Captured products keep no partial sums: replays of two graphs may overlap, on
+    // other streams than the library's, and would share the buffer.  One CTA
     // then takes all parts of its block, us outside / inside a graph / tiled kernel there:
     // sparse SYK, complex128, 12 qubits 6.1 / 10.2 / 49, 14 qubits 7.5 / 11.7 / 86; dense SYK,
     // 8 qubits 6.6 / 29 / 377, 12 qubits 16.7 / 117 / 2283.
@@ -350,6 +371,9 @@ static void launch_runs(const RunPlan &p, const RunLaunch &l, cudaStream_t st) {
     if (p.parts > 1) RP_CUDA(cudaStreamIsCapturing(st, &capture));
     a.span = capture == cudaStreamCaptureStatusNone ? 1 : p.parts;
     a.parts = p.parts / a.span;
+    char *const shared = a.parts > 1 ? runs_scratch() : nullptr;
+    a.partial = reinterpret_cast<Cplx<Real> *>(shared);
+    a.arrived = shared ? reinterpret_cast<unsigned *>(shared + runs_partial_bytes()) : nullptr;
     a.dim = (size_t)p.nblocks * (32u << EB);
     a.alpha = l.alpha;
     a.alpha_dev = l.alpha_dev;

@@ -27,19 +27,14 @@ struct TablePack {
     std::vector<uint8_t> bytes;
     template <typename T>
     size_t add(const std::vector<T> &v) {
-        const size_t at = room(v.size() * sizeof(T));
+        const size_t at = bytes.size();
+        bytes.resize(at + ((v.size() * sizeof(T) + 15) & ~size_t(15)), 0);
         if (!v.empty()) std::memcpy(bytes.data() + at, v.data(), v.size() * sizeof(T));
         return at;
     }
-    size_t room(size_t n) {              // n zero bytes
-        const size_t at = bytes.size();
-        bytes.resize(at + ((n + 15) & ~size_t(15)), 0);
-        return at;
-    }
-    // the tables on the device, `scratch` bytes that are not copied after them
-    char *upload(size_t scratch = 0) const {
+    char *upload() const {               // the tables on the device
         void *d = nullptr;
-        RP_CUDA(cudaMalloc(&d, bytes.size() + scratch + 16));
+        RP_CUDA(cudaMalloc(&d, bytes.size() + 16));
         const cudaError_t e = cudaMemcpy(d, bytes.data(), bytes.size(), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) cudaFree(d);
         RP_CUDA(e);
@@ -55,19 +50,18 @@ struct RunPlan {
     std::vector<RunTerm> terms;
     std::vector<Run> runs;               // cut at the workers' boundaries
     std::vector<uint32_t> wstart;        // worker -> first run (workers + 1 entries)
-    // one allocation: terms, runs, wstart, and (parts > 1) the parts' partial
-    // sums and the blocks' arrival counts, for the launches on the library's stream,
-    // which run one after the other (captured ones do without: launch_runs)
-    char *dev = nullptr;
-    size_t at_runs = 0, at_wstart = 0, at_arrived = 0, at_partial = 0;
+    char *dev = nullptr;                 // one allocation: terms, runs, wstart
+    size_t at_runs = 0, at_wstart = 0;
 };
 
 constexpr int RUN_MIN_LEN = 5;           // smaller states: the direct kernel
 
 // Host only: sort the terms into runs and deal them out to the workers.
 void runplan_build(RunPlan &p, int len, const uint64_t *bits, const double *coeff, int64_t nterms);
-void runplan_upload(RunPlan &p, int len, int dtype);
+void runplan_upload(RunPlan &p);
 void runplan_free(RunPlan &p);
+// The partial sums that all plans share (rp_shutdown).
+void runs_scratch_release();
 
 struct RunLaunch {
     const void *in = nullptr;

@@ -151,6 +151,7 @@ int rp_shutdown(void) {
         krylov_scratch_release();
         pipe_release();
         scratch_release_all();
+        runs_scratch_release();
         dense_handles_release();
         if (g_dev_err) cudaFree(g_dev_err);
         g_dev_err = nullptr;
