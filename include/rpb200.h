@@ -49,7 +49,8 @@ typedef struct {
     int grid;            /* persistent CTAs */
     double alg_bytes;    /* (ngroups + 1) * 2^len * element size per apply */
     int kernel;          /* 0 direct, 1 tiled (bulk copies), 2 rows (TMA, swizzled),
-                          * 3 split rows (a cluster per tile), 4 runs (small states);
+                          * 3 split rows (a cluster per tile), 4 runs (a gather per X
+                          * mask: smaller states, lists too long for the row kernel);
                           * for 3 and 4 the byte figures are the tiled kernel's */
     int window;          /* CTAs in flight = aligned block of output tiles */
     double alg_bytes_dram; /* (G_w + 1) * 2^len * element size, G_w = distinct

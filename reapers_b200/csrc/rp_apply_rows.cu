@@ -39,8 +39,9 @@
 // terms of an X mask with equal chunk signs (a bond's XX and YY) are summed to
 // one coefficient per row first, a record says whether the next one belongs to
 // it, and the part of the diagonal without a Z bit in the tile is summed over the
-// lanes, once per tile.  XXZ chain: 2^27 complex64 2.66 -> 2.53 ms (2.77 with the
-// divisions), 2^26 complex128 2.67 -> 2.45 (2.80), 2^24 complex128 0.619 -> 0.579.
+// lanes, once per tile.  XXZ chain: 2^27 complex64 2.66 -> 2.53 to 2.64 ms, by the box
+// (2.77 with the divisions), 2^26 complex128 2.67 -> 2.45 (2.80), 2^24 complex128 0.619 ->
+// 0.579.
 // Dealing the bonds out to passes over strided tiles instead, one load of input
 // and output per 8 index bits, moved half the bytes and gave 2.47 ms, and with a
 // third ring stage given up for a diagonal kept per row 2.63: left out.

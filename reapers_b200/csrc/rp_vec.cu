@@ -159,8 +159,9 @@ void vec_random(int dtype, uint64_t n, void *v, uint64_t seed, cudaStream_t st) 
 constexpr int RT = 256;   // threads of the reduction kernels
 constexpr int RW = RT / 32;
 
-// <a|b>: a CTA sums every gridDim-th stretch of packets, four loads of each
-// vector in flight per thread; the last CTA to arrive adds the CTAs' partials
+// <a|b> (a norm is <v|v>, its second load of a packet served by L1): a CTA sums
+// every gridDim-th stretch of packets, four loads of each vector in flight per
+// thread; the last CTA to arrive adds the CTAs' partials
 // (compensated, fixed order) and writes the pair to pinned host memory, so a
 // call is one launch and one synchronisation.  (Two kernels, the second adding
 // 296 partials in one thread, and a copy: 30 us on the device for 2^16
@@ -268,8 +269,8 @@ double vec_norm(int dtype, uint64_t n, const void *v, cudaStream_t st) {
     return std::sqrt(out[0]);
 }
 
-// w += sum_i c_i u_i in one pass: per packet of w, the vectors
-// are read in groups of AXPY_G independent 16-byte loads, the update is
+// w += sum_i c_i u_i in one pass: per packet of w, the vectors are read in
+// groups of eight independent 16-byte loads (axpy_vectors), the update is
 // accumulated in FP64 and rounded once to the vector precision.
 template <typename Real>
 __global__ void __launch_bounds__(RT) k_multi_axpy(uint64_t npk, const VecTable tab, int nvec,

@@ -14,8 +14,9 @@ struct VecTable {
 };
 
 // Vectors are streamed as 16-byte packets: one complex double or two complex
-// floats.  A packet count of n * sizeof(element) / 16 requires an even n for
-// complex64; the element-wise kernels further down handle the odd case.
+// floats.  A packet count of n * sizeof(element) / 16 leaves out the last element
+// of an odd complex64 vector; k_dot adds it, the others take states, whose length
+// is even.
 template <typename Real>
 struct Packet;
 template <>
@@ -120,10 +121,9 @@ double vec_norm(int dtype, uint64_t n, const void *v, cudaStream_t st);
 void multi_axpy(int dtype, uint64_t n, const VecTable &tab, int nvec, const int *nvec_dev,
                 const double *coef, void *w, cudaStream_t st);
 
-// Device scratch kept between calls: the step-size candidates' expm buffer, the dense
-// matrix-vector product's column-chunk partials and the dense exponential's
-// scaled eigenvectors.  A slot
-// grows on demand (the stream is synchronised before a smaller buffer is
+// Device scratch kept between calls: the step-size candidates' expm buffer, the
+// dense matrix-vector product's column-chunk partials and the dense exponential's
+// scaled eigenvectors.  A slot grows on demand (the stream is synchronised before a smaller buffer is
 // freed); scratch_release_all(), called by rp_shutdown, frees every slot, so
 // a later rp_init allocates them afresh.
 enum ScratchSlot { SCR_EXPM = 0, SCR_MATVEC, SCR_EXPM_DENSE, SCR_COUNT };
